@@ -210,7 +210,9 @@ def prepare(case, seed):
         s["engine"] = BatchEngine(_batch(case, seed), case["precision"], tile_bits=case["tile_bits"],
                                   ctas_per_sm=case["ctas"])
         s["out"] = torch.empty(s["engine"].rho_elems, dtype=torch.complex128,
-                               pin_memory=torch.cuda.is_available()).numpy()
+                               pin_memory=torch.cuda.is_available())
+        if case["precision"] == 1:
+            s["single"] = torch.empty(s["engine"].rho_elems, dtype=torch.complex64)
         return s
     if kind == "join":
         rng = _rng(case, seed)
@@ -266,8 +268,8 @@ def run(state):
     d, case, kind = s["d"], s["case"], s["kind"]
     if kind == "batch":
         s["engine"].run()
-        out, _ = s["engine"].rho_all(s["out"])
-        return _complex(case, out)
+        s["engine"].rho_all(s["out"].numpy())
+        return s["single"].copy_(s["out"]) if case["precision"] == 1 else s["out"]
     if kind == "join":
         reg = d.registry_join(s["most"], s["least"], -1, False)
         return _real(case, d.registry_probs(reg))
