@@ -1435,25 +1435,21 @@ __global__ void k_clear_flags(dk_scal *sc)
  * in registers).  Two 256-thread blocks fit per SM. */
 constexpr int kMargHi = 24;
 
-/* Block sum of v into partials[slot] (thread 0), uniform call sites only. */
-__device__ __forceinline__ void marg_store(double v, double *red, double *dst)
+/* Sum over the warp, in every lane (fixed order). */
+__device__ __forceinline__ double warp_sum(double v)
 {
-	const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
 #pragma unroll
 	for (int o = 16; o > 0; o >>= 1)
 		v += __shfl_xor_sync(0xffffffffu, v, o);
-	if (l == 0)
-		red[w] = v;
-	__syncthreads();
-	if (threadIdx.x == 0) {
-		double t = 0.0;
-		for (int i = 0; i < (int)(blockDim.x >> 5); ++i)
-			t += red[i];
-		*dst = t;
-	}
-	__syncthreads();
+	return v;
 }
 
+/* Bound by the read of the register.  The block's n + 1 sums are taken
+ * together: each warp sums tot, tot over the lanes with lane bit b set, and
+ * every acc[j] with shuffles, and one thread per qubit adds the 8 warps' values
+ * (warp bits and block bits of g select whole warps' totals), with a single
+ * block barrier.  A block sum per qubit, two barriers each, took 41 of the
+ * 124 us of a 24-qubit complex128 launch. */
 template <typename R, int NB>
 __global__ void __launch_bounds__(256, 2)
 	k_marginals(const typename CT<R>::T *__restrict__ d, int n, int s,
@@ -1505,27 +1501,65 @@ __global__ void __launch_bounds__(256, 2)
 					acc[j] += p;
 		}
 	}
-	__shared__ double red[32];
-	double *const out = partials + (size_t)blockIdx.x * kPartialStride;
-	/* q < s: tot * bit_q(g); q = s + j: acc[j]; q = n: tot */
-	for (int q = 0; q < s && q < n; ++q)
-		marg_store(((g >> q) & 1u) ? tot : 0.0, red, out + q);
+	/* per warp: total, the 5 lane-bit sums, the NB loop-bit sums */
+	__shared__ double red[8][6 + NB];
+	const uint32_t w = threadIdx.x >> 5, l = threadIdx.x & 31u;
+	double v = warp_sum(tot);
+	if (l == 0)
+		red[w][0] = v;
+#pragma unroll
+	for (int b = 0; b < 5; ++b) {
+		v = warp_sum(((l >> b) & 1u) ? tot : 0.0);
+		if (l == 0)
+			red[w][1 + b] = v;
+	}
 #pragma unroll
 	for (int j = 0; j < NB; ++j)
-		if (j < nb)
-			marg_store(acc[j], red, out + s + j);
-	marg_store(tot, red, out + n);
-}
-
-__global__ void k_marg_finalize(const double *partials, int nb, int n, double *marg)
-{
-	const int q = threadIdx.x;
+		if (j < nb) {
+			v = warp_sum(acc[j]);
+			if (l == 0)
+				red[w][6 + j] = v;
+		}
+	__syncthreads();
+	/* q < s: tot over the threads whose g has bit q; q = s + j: acc[j];
+	 * q = n: tot (blocks have at least n + 1 threads, see the launcher) */
+	const int q = (int)threadIdx.x;
 	if (q > n)
 		return;
+	int col = 0;
+	uint32_t wmask = 0; /* warps whose index has this bit, 0: every warp */
+	bool none = false;
+	if (q == n)
+		col = 0;
+	else if (q >= s)
+		col = 6 + q - s;
+	else if (q < 5)
+		col = 1 + q;
+	else if (q < 8)
+		wmask = 1u << (q - 5);
+	else
+		none = !((blockIdx.x >> (q - 8)) & 1u);
 	double t = 0.0;
-	for (int b = 0; b < nb; ++b)
+	if (!none)
+		for (uint32_t i = 0; i < (blockDim.x >> 5); ++i)
+			if ((i & wmask) == wmask)
+				t += red[i][col];
+	partials[(size_t)blockIdx.x * kPartialStride + q] = t;
+}
+
+/* marg[q] = sum of the blocks' partials, in a fixed order: one block per
+ * qubit (one thread per qubit took 136 us for the 2048 partials of a 24-qubit
+ * register, longer than the pass over the register itself; this takes 5). */
+__global__ void __launch_bounds__(256)
+	k_marg_finalize(const double *partials, int nb, double *marg)
+{
+	const int q = blockIdx.x;
+	double t = 0.0, dummy = 0.0;
+	for (int b = threadIdx.x; b < nb; b += blockDim.x)
 		t += partials[(size_t)b * kPartialStride + q];
-	marg[q] = t;
+	block_sum2(dummy, t);
+	if (threadIdx.x == 0)
+		marg[q] = t;
 }
 
 /* ---- measurement -------------------------------------------------------- */
@@ -2609,7 +2643,7 @@ cudaError_t launch_marginals(int prec, const void *d, unsigned n, const Scratch 
 		sbits = (int)n;
 	}
 	launch_marginals_kernel(prec, d, n, sbits, blocks, threads, s.partials, st);
-	k_marg_finalize<<<1, 64, 0, st>>>(s.partials, blocks, (int)n, s.marg);
+	k_marg_finalize<<<n + 1, 256, 0, st>>>(s.partials, blocks, s.marg);
 	g_launches += 2;
 	return cudaGetLastError();
 }
@@ -2656,8 +2690,8 @@ cudaError_t launch_marginals_blocks(int prec, const void *d, unsigned n,
 	if (e != cudaSuccess)
 		return e;
 	int nblk = blocks;
-	void *fargs[] = { (void *)&partials, (void *)&nblk, (void *)&ni, (void *)&marg };
-	e = cudaLaunchKernel((const void *)k_marg_finalize, dim3(1), dim3(64), fargs, 0, st);
+	void *fargs[] = { (void *)&partials, (void *)&nblk, (void *)&marg };
+	e = cudaLaunchKernel((const void *)k_marg_finalize, dim3(n + 1), dim3(256), fargs, 0, st);
 	g_launches += (e == cudaSuccess) ? 2 : 1;
 	return e;
 }
