@@ -1636,151 +1636,174 @@ __device__ __forceinline__ uint64_t deposit_mask(uint64_t v, uint64_t mask)
 	return out;
 }
 
-/* partials[bin * nchunk + c] = sum of |amp|^2 over chunk c of the bin */
+/* Joint distribution of the k measured qubits, bound by one read of the
+ * register.  The register is read in contiguous chunks of 2^c amplitudes
+ * (c = min(n, 12)); block row y takes the chunks whose index has the y-th
+ * pattern of the measured qubits at or above c, split over the blocks x of
+ * the row.  Thread t adds up position t + 256 u of every chunk in the register
+ * acc[u], so the loop knows nothing of bins: the measured qubits below c are
+ * told apart once per block, when the 16 x 256 sums are added into its 2^kl
+ * bins (in a fixed order).  Every read is coalesced and used once whatever the
+ * mask.  Blocks per bin that gather the bin's amplitudes read part of each
+ * 32-byte sector when a low qubit is measured, and walk the deposit table per
+ * amplitude: 688 us for 7 scattered qubits of 27 (complex128), 2.1 GB.
+ *
+ * partials[bin * gridDim.x + x], bin = low bins | pattern << kl. */
+constexpr int kJointChunkBits = 12;
+
 template <typename R>
 __global__ void __launch_bounds__(256)
-	k_joint(const typename CT<R>::T *__restrict__ in, DepRuns runs, uint64_t mask,
-		uint64_t per_bin, uint64_t chunk, uint64_t nchunk, double *partials)
+	k_joint(const typename CT<R>::T *__restrict__ in, int c, uint32_t lmask, uint64_t hmask,
+		uint64_t hfree, uint64_t nchunk, uint64_t per_block,
+		[[maybe_unused]] uint64_t size, double *partials)
 {
-	__shared__ DepRuns sr;
-	if (threadIdx.x == 0)
-		sr = runs;
-	__syncthreads();
-	const uint64_t bin = blockIdx.y;
-	const uint64_t vb = deposit_mask(bin, mask);
-	[[maybe_unused]] const uint64_t nin = per_bin << __popcll(mask);
-	for (uint64_t c = blockIdx.x; c < nchunk; c += gridDim.x) {
-		double sum = 0.0, dummy = 0.0;
-		const uint64_t j0 = c * chunk;
-		uint64_t j1 = j0 + chunk;
-		if (j1 > per_bin)
-			j1 = per_bin;
-		for (uint64_t j = j0 + threadIdx.x; j < j1; j += blockDim.x) {
-			const uint64_t i = dep_runs(sr, j) | vb;
-			if (DK_IN_BOUNDS(i, nin, CHK_JOINT))
-				sum += sqabs(__ldcs(in + i));
+	__shared__ double hist[16 * 256];
+	__shared__ double red[256];
+	const uint32_t t = threadIdx.x;
+	double acc[16];
+#pragma unroll
+	for (int u = 0; u < 16; ++u)
+		acc[u] = 0.0;
+	const uint64_t pat = deposit_mask(blockIdx.y, hmask);
+	const uint64_t j0 = (uint64_t)blockIdx.x * per_block;
+	uint64_t j1 = j0 + per_block;
+	if (j1 > nchunk)
+		j1 = nchunk;
+	const uint32_t cnt = 1u << c;
+	if (j0 < j1) {
+		uint64_t high = deposit_mask(j0, hfree);
+		for (uint64_t j = j0; j < j1; ++j) {
+			const uint64_t base = ((high | pat) << c) + t;
+			if (cnt == 4096u) {
+				double p[16];
+#pragma unroll
+				for (int u = 0; u < 16; ++u)
+					p[u] = DK_IN_BOUNDS(base + 256u * u, size, CHK_JOINT)
+						       ? sqabs(__ldcs(in + base + 256u * u))
+						       : 0.0;
+#pragma unroll
+				for (int u = 0; u < 16; ++u)
+					acc[u] += p[u];
+			} else {
+#pragma unroll
+				for (int u = 0; u < 16; ++u)
+					if (t + 256u * u < cnt &&
+					    DK_IN_BOUNDS(base + 256u * u, size, CHK_JOINT))
+						acc[u] += sqabs(__ldcs(in + base + 256u * u));
+			}
+			/* the next index of the unmeasured high qubits */
+			high = (high - hfree) & hfree;
 		}
-		block_sum2(dummy, sum);
-		if (threadIdx.x == 0)
-			partials[bin * nchunk + c] = sum;
+	}
+#pragma unroll
+	for (int u = 0; u < 16; ++u)
+		hist[256 * u + t] = acc[u];
+	__syncthreads();
+	/* bin b: the members are the positions of the chunk with the measured
+	 * bits of b, one for each value of the unmeasured bits */
+	const uint32_t free_bits = (cnt - 1u) & ~lmask;
+	const int kl = __popc(lmask);
+	const uint32_t nb = 1u << kl, members = cnt >> kl;
+	const uint64_t out = ((uint64_t)blockIdx.y << kl) * gridDim.x + blockIdx.x;
+	if (nb >= 256u) {
+		for (uint32_t b = t; b < nb; b += 256u) {
+			const uint32_t fix = (uint32_t)deposit_mask(b, lmask);
+			uint32_t f = 0;
+			double v = 0.0;
+			for (uint32_t i = 0; i < members; ++i) {
+				v += hist[fix | f];
+				f = (f - free_bits) & free_bits;
+			}
+			partials[out + (uint64_t)b * gridDim.x] = v;
+		}
+		return;
+	}
+	/* 256 / nb threads per bin, added up in pairs */
+	const uint32_t g = 256u >> kl, gi = t & (g - 1u), b = t / g;
+	const uint32_t each = members / g;
+	const uint32_t fix = (uint32_t)deposit_mask(b, lmask);
+	double v = 0.0;
+	if (each) {
+		uint32_t f = (uint32_t)deposit_mask((uint64_t)gi * each, free_bits);
+		for (uint32_t i = 0; i < each; ++i) {
+			v += hist[fix | f];
+			f = (f - free_bits) & free_bits;
+		}
+	} else if (gi < members) {
+		v = hist[fix | (uint32_t)deposit_mask(gi, free_bits)];
+	}
+	red[t] = v;
+	__syncthreads();
+	for (uint32_t st = g >> 1; st > 0; st >>= 1) {
+		if (gi < st)
+			red[t] += red[t + st];
 		__syncthreads();
 	}
+	if (gi == 0)
+		partials[out + (uint64_t)b * gridDim.x] = red[t];
 }
 
-/* Joint distribution of k <= 4 measured qubits in one contiguous pass over
- * the register (coalesced like k_marginals): thread t adds |amp_i|^2 to its
- * own shared-memory column hist[bin(i)][t], no atomics, and the columns of
- * each bin are added in a fixed order.  Writes partials[bin * gridDim.x +
- * block] as k_joint does, for k_joint_finalize.  k_joint instead gives each
- * bin its own blocks, which gather the bin's amplitudes; with a low measured
- * qubit those gathers use part of every 32-byte sector and every bin re-reads
- * the same sectors. */
-constexpr int kJointSmallBins = 16;
-constexpr uint64_t kJointSeg = 4096; /* amplitudes per block step, 16 per thread */
-
-template <typename R>
+/* joint[bin] = sum of its blocks, a warp per bin, in a fixed order */
 __global__ void __launch_bounds__(256)
-	k_joint_small(const typename CT<R>::T *__restrict__ in, uint64_t size, uint32_t qpack,
-		      int k, double *partials)
+	k_joint_finalize(const double *partials, uint64_t nsplit, uint32_t nbins, double *joint)
 {
-	__shared__ double hist[kJointSmallBins][256];
-	const uint32_t t = threadIdx.x;
-	const int nb = 1 << k;
-	for (int b = 0; b < nb; ++b)
-		hist[b][t] = 0.0; /* each thread only ever touches its own column */
-	int qs[4];
-#pragma unroll
-	for (int j = 0; j < 4; ++j)
-		qs[j] = (int)((qpack >> (8 * j)) & 0xffu);
-	for (uint64_t base = (uint64_t)blockIdx.x * kJointSeg; base < size;
-	     base += (uint64_t)gridDim.x * kJointSeg) {
-		double p[16];
-#pragma unroll
-		for (int u = 0; u < 16; ++u)
-			p[u] = DK_IN_BOUNDS(base + t + 256u * u, size, CHK_JOINT)
-				       ? sqabs(__ldcs(in + base + t + 256u * u))
-				       : 0.0;
-#pragma unroll
-		for (int u = 0; u < 16; ++u) {
-			const uint64_t i = base + t + 256u * u;
-			uint32_t b = 0;
-#pragma unroll
-			for (int j = 0; j < 4; ++j)
-				if (j < k)
-					b |= (uint32_t)((i >> qs[j]) & 1u) << j;
-			hist[b][t] += p[u];
-		}
-	}
-	__syncthreads();
-	const uint32_t w = t >> 5, l = t & 31u;
-	for (int b = (int)w; b < nb; b += (int)(blockDim.x >> 5)) {
-		double v = 0.0;
-		for (uint32_t c = l; c < 256u; c += 32u)
-			v += hist[b][c];
-#pragma unroll
-		for (int o = 16; o > 0; o >>= 1)
-			v += __shfl_xor_sync(0xffffffffu, v, o);
-		if (l == 0)
-			partials[(uint64_t)b * gridDim.x + blockIdx.x] = v;
-	}
+	const uint32_t bin = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, l = threadIdx.x & 31u;
+	if (bin >= nbins)
+		return;
+	double sum = 0.0;
+	for (uint64_t c = l; c < nsplit; c += 32)
+		sum += partials[bin * nsplit + c];
+	sum = warp_sum(sum);
+	if (l == 0)
+		joint[bin] = sum;
 }
 
-/* joint[bin] = sum of its chunks, in order */
-__global__ void __launch_bounds__(256)
-	k_joint_finalize(const double *partials, uint64_t nchunk, double *joint)
-{
-	double sum = 0.0, dummy = 0.0;
-	for (uint64_t c = threadIdx.x; c < nchunk; c += blockDim.x)
-		sum += partials[blockIdx.x * nchunk + c];
-	block_sum2(dummy, sum);
-	if (threadIdx.x == 0)
-		joint[blockIdx.x] = sum;
-}
-
-/* One warp: outcomes of the k measured qubits, highest first, from the
+/* One block: outcomes of the k measured qubits, highest first, from the
  * joint distribution; flags[s] = outcome of step s; *vbits = the outcomes
  * deposited into the measured positions; sc_out->p_sel = probability of the
- * whole outcome relative to the stored norm. */
-__global__ void k_decide_joint(const double *joint, int k, const double *rolls, int32_t *flags,
-			       uint64_t *vbits, uint64_t mask, const dk_scal *sc_in,
-			       dk_scal *sc_out)
+ * whole outcome relative to the stored norm.  The sums over the bins that
+ * share their j highest bits are the nodes of a binary tree (children 2 i and
+ * 2 i + 1, bins below the last level), built level by level by all threads;
+ * the decisions then walk it from the root.  One warp adding up the bins left
+ * at every step took 122 us for 12 qubits, bound by the latency of k passes
+ * over 4096 bins; the tree takes 11. */
+__global__ void __launch_bounds__(256)
+	k_decide_joint(const double *joint, int k, const double *rolls, int32_t *flags,
+		       uint64_t *vbits, uint64_t mask, const dk_scal *sc_in, dk_scal *sc_out)
 {
-	const uint32_t lane = threadIdx.x;
-	const uint32_t nb = 1u << k;
+	__shared__ double node[1 << kJointMaxQubits];
+	for (uint32_t i = threadIdx.x; i < (1u << (k - 1)); i += blockDim.x)
+		node[(1u << (k - 1)) + i] = joint[2 * i] + joint[2 * i + 1];
+	__syncthreads();
+	for (int lev = k - 2; lev >= 0; --lev) {
+		for (uint32_t i = threadIdx.x; i < (1u << lev); i += blockDim.x) {
+			const uint32_t x = (1u << lev) + i;
+			node[x] = node[2 * x] + node[2 * x + 1];
+		}
+		__syncthreads();
+	}
+	if (threadIdx.x != 0)
+		return;
 	/* the first probability is relative to the stored norm, as the
 	 * reference's (data registers need not be normalised); the later ones
 	 * are conditional on the outcomes so far */
 	const double n2 = sc_in->norm * sc_in->norm;
-	uint32_t pm = 0, pv = 0;
 	double prev = n2;
+	uint32_t at = 1;
 	for (int st = 0; st < k; ++st) {
-		const int bb = k - 1 - st; /* bin bit of the qubit measured now */
-		double s1 = 0.0, s0 = 0.0;
-		for (uint32_t b = lane; b < nb; b += 32)
-			if ((b & pm) == pv) {
-				if ((b >> bb) & 1u)
-					s1 += joint[b];
-				else
-					s0 += joint[b];
-			}
-		for (int o = 16; o > 0; o >>= 1) {
-			s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-			s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-		}
+		const bool last = st == k - 1;
+		const uint32_t c = 2 * at, lb = c - (1u << k);
+		const double s0 = last ? joint[lb] : node[c], s1 = last ? joint[lb + 1] : node[c + 1];
 		const double p = prev > 0.0 ? s1 / prev : 0.0;
 		const int res = p > rolls[st] ? 1 : 0;
-		pm |= 1u << bb;
-		pv |= (uint32_t)res << bb;
 		prev = res ? s1 : s0;
-		if (lane == 0)
-			flags[st] = res;
+		at = c + (uint32_t)res;
+		flags[st] = res;
 	}
-	if (lane == 0) {
-		*vbits = deposit_mask(pv, mask);
-		sc_out->flag = 0;
-		sc_out->p_sel = n2 > 0.0 ? prev / n2 : 0.0;
-		sc_out->zero_norm = 0;
-	}
+	*vbits = deposit_mask(at - (1u << k), mask);
+	sc_out->flag = 0;
+	sc_out->p_sel = n2 > 0.0 ? prev / n2 : 0.0;
+	sc_out->zero_norm = 0;
 }
 
 /* out[j] = in[j deposited into the unmeasured positions | measured bits] */
@@ -2747,47 +2770,35 @@ cudaError_t launch_measure_joint(int prec, const void *in, void *out, unsigned n
 		src += e - q;
 		q = e;
 	}
-	const uint64_t nbins = 1ull << k, per_bin = 1ull << (n - k);
-	/* chunks of >= 4096 amplitudes, at most kJointPartials partials */
-	uint64_t nchunk = (per_bin + 4095) / 4096;
-	if (nchunk * nbins > kJointPartials)
-		nchunk = kJointPartials / nbins;
-	if (nchunk < 1)
-		nchunk = 1;
-	const uint64_t chunk = (per_bin + nchunk - 1) / nchunk;
+	const uint64_t nbins = 1ull << k, per_bin = 1ull << (n - k), size = 1ull << n;
 	double *part = s.partials;
 	double *joint = s.partials + kJointPartials;
 	uint64_t *vbits = reinterpret_cast<uint64_t *>(s.u64 + 1);
-	if (k <= 4 && n >= 12) {
-		/* one contiguous pass, 2048 blocks at most */
-		uint32_t qpack = 0;
-		int j = 0;
-		for (unsigned q = 0; q < n; ++q)
-			if ((mask >> q) & 1u)
-				qpack |= q << (8 * j++);
-		const uint64_t size = 1ull << n;
-		uint64_t nb = size / kJointSeg;
-		if (nb > 2048)
-			nb = 2048;
-		if (prec == DK_C128)
-			k_joint_small<double><<<(unsigned)nb, 256, 0, st>>>((const double2 *)in, size,
-									    qpack, k, part);
-		else
-			k_joint_small<float><<<(unsigned)nb, 256, 0, st>>>((const float2 *)in, size,
-									   qpack, k, part);
-		k_joint_finalize<<<(unsigned)nbins, 256, 0, st>>>(part, nb, joint);
-	} else {
-		uint64_t gx = nchunk < (uint64_t)g_num_sms * 8 ? nchunk : (uint64_t)g_num_sms * 8;
-		dim3 grid((unsigned)gx, (unsigned)nbins);
-		if (prec == DK_C128)
-			k_joint<double><<<grid, 256, 0, st>>>((const double2 *)in, runs, mask,
-							      per_bin, chunk, nchunk, part);
-		else
-			k_joint<float><<<grid, 256, 0, st>>>((const float2 *)in, runs, mask,
-							     per_bin, chunk, nchunk, part);
-		k_joint_finalize<<<(unsigned)nbins, 256, 0, st>>>(part, nchunk, joint);
-	}
-	k_decide_joint<<<1, 32, 0, st>>>(joint, k, rolls_dev, flags_dev, vbits, mask, sc_in, sc_out);
+	const int c = (int)n < kJointChunkBits ? (int)n : kJointChunkBits;
+	const uint64_t hmask = mask >> c, hfree = ((size >> c) - 1ull) & ~hmask;
+	const uint64_t rows = 1ull << __builtin_popcountll(hmask);
+	const uint64_t nchunk = 1ull << __builtin_popcountll(hfree); /* per row */
+	/* about 2048 blocks (7 waves of two per SM at 30 qubits), within the
+	 * scratch for their partials */
+	uint64_t nsplit = 2048 / rows;
+	if (nsplit > kJointPartials / nbins)
+		nsplit = kJointPartials / nbins;
+	if (nsplit > nchunk)
+		nsplit = nchunk;
+	if (nsplit < 1)
+		nsplit = 1;
+	const uint64_t per_block = (nchunk + nsplit - 1) / nsplit;
+	const dim3 grid((unsigned)nsplit, (unsigned)rows);
+	const uint32_t lmask = (uint32_t)(mask & ((1ull << c) - 1ull));
+	if (prec == DK_C128)
+		k_joint<double><<<grid, 256, 0, st>>>((const double2 *)in, c, lmask, hmask, hfree,
+						      nchunk, per_block, size, part);
+	else
+		k_joint<float><<<grid, 256, 0, st>>>((const float2 *)in, c, lmask, hmask, hfree,
+						     nchunk, per_block, size, part);
+	k_joint_finalize<<<(unsigned)((nbins + 7) / 8), 256, 0, st>>>(part, nsplit, (uint32_t)nbins,
+								      joint);
+	k_decide_joint<<<1, 256, 0, st>>>(joint, k, rolls_dev, flags_dev, vbits, mask, sc_in, sc_out);
 	g_launches += 3;
 	if (out != nullptr) {
 		const int blocks = grid_for(per_bin, 256 * 4, g_num_sms * 8);
