@@ -189,7 +189,93 @@ typedef struct dk_sweep_hdr {
  * by per-thread FP arithmetic on 8 register amplitudes.  TENSOR: every entry
  * is an 8x8 matrix in register order (controls on non-pass tile bits and
  * outside the tile in the descriptor), applied with FP64 tensor-core MMAs. */
-enum { DK_SWEEP_SCALAR = 0, DK_SWEEP_TENSOR = 1 };
+enum { DK_SWEEP_SCALAR = 0, DK_SWEEP_TENSOR = 1, DK_SWEEP_FACTORED = 2 };
+
+/* ---- factored sweeps -----------------------------------------------------
+ * A pass gathers, per thread, the 16 amplitudes that differ in 4 tile bits.
+ * Its gates are factored on the host into operations on those registers:
+ *  - a one-qubit gate U = diag(l0, l1) [[1, -s], [t, 1]] diag(1, r1) with real
+ *    s and t (every unitary has this form): one real multiply-add per
+ *    amplitude component instead of the four of a complex 2x2 product;
+ *  - diagonal factors, collected over all gates of a stage into one product;
+ *  - X and CNOT, which only relabel the registers: register p holds the
+ *    amplitude of pass index L(p), L affine over GF(2), and the scatter writes
+ *    it to that index's slot.
+ * Qubits outside the tile that condition a gate select one of the pass's
+ * 2^ncond operation lists.  Everything is stored in the amplitude precision. */
+#define DK_FX_BITS 4
+#define DK_FX_REGS 16
+#define DK_FX_COND 3 /* most tile conditions of a pass */
+#define DK_FX_MIN_TILE 9 /* tile bits: a full warp of 16-amplitude columns */
+#define DK_FX_MAX_GATES 512 /* gates of a sweep */
+#define DK_MAX_FX_PASSES DK_FX_MAX_GATES
+/* Most bytes of a factored program, which the kernel keeps in shared memory:
+ * two CTAs with a 64 KiB (three with a 32 KiB) tile each share an SM; a
+ * register of few tiles has one CTA per SM and takes longer programs instead of
+ * more sweeps. */
+#define DK_FX_BYTES (40u << 10)
+#define DK_FX_BYTES_SMALL (140u << 10)
+#define DK_FX_SMALL_TILES 7 /* log2 of the most tiles for a long program */
+
+/* Operation (16 bytes), on the registers a[0..16) of a thread; v is a
+ * direction 1..15, its pairs are (p, q = p ^ v) for the 8 p without the lowest
+ * bit of v, in increasing order.
+ *   DK_FX_STAGE     coefficients: four real pairs (x, y), complex64 (x, x, y, y),
+ *                   then, with mask bit 4, 16 complex values.  Mask bit 4: a[p] *=
+ *                   value p; then for each mask bit j < 4, the pairs of
+ *                   direction 1 << j: a[p] += x a[q], a[q] += y a[p] (old
+ *                   values) with pair j
+ *   DK_FX_ROT + v   the pairs of direction v, each with its own (x, y)
+ *   DK_FX_PHASE     a[p] *= coefs[0] for the p in mask
+ *   DK_FX_NEG       a[p] = -a[p] for the p in mask
+ *   DK_FX_SWAP + v  a[p] <-> a[q] for the pairs in mask
+ * lc / la: control / anticontrol masks over the tile bits outside the pass. */
+enum {
+	DK_FX_STAGE = 0,
+	DK_FX_ROT = 0, /* + 1..15 */
+	DK_FX_PHASE = 16,
+	DK_FX_SWAP = 16, /* + 1..15 */
+	DK_FX_NEG = 32,
+};
+typedef struct dk_fx_op {
+	uint16_t code;
+	uint16_t mask;
+	uint32_t coef; /* 16-byte units from the coefficient table */
+	uint32_t lc, la;
+} dk_fx_op;
+
+/* What a pass does where its tile conditions have one combination of values:
+ * operations [op0, op1) between a gather and a scatter, whose slots are given
+ * by byte offsets for register bit j and for register 0 (relabellings move
+ * amplitudes in between, and the gather may choose the labels). */
+typedef struct dk_fx_list {
+	uint16_t gt[DK_FX_BITS], st[DK_FX_BITS];
+	uint16_t gc, sc;
+	uint16_t op0, op1;
+	/* the scatter as pass indices: L(1 << j) ^ L(0) in nibble j, L(0) in
+	 * nibble 4 (a pass that stores to the register) */
+	uint32_t lmap;
+	uint32_t idle; /* nothing to do */
+} dk_fx_list; /* 32 bytes */
+
+typedef struct dk_fx_pass {
+	uint32_t flags; /* DK_PASS_WARP, DK_PASS_CTL, DK_FX_STORE */
+	uint32_t list; /* its first list; 2^ncond follow each other */
+	/* indices of its tile conditions, 5 bits each, their number in bits 15-16;
+	 * condition j holding adds 2^j to the list */
+	uint32_t cond;
+	uint32_t pad;
+	uint16_t pm[DK_FX_BITS]; /* raw tile-index mask of pass bit j */
+	uint16_t shi[8], slo[32]; /* byte offsets of thread bits 5-7 / 0-4 */
+	uint16_t rhi[8], rlo[32]; /* raw tile-index bits of the same */
+	uint16_t pad2[4];
+} dk_fx_pass; /* 192 bytes; a program's lists follow its passes */
+
+#define DK_FX_MAX_CONDS 32 /* tile conditions of a program: one per lane */
+
+/* The last pass of a sweep, when its lanes carry the tile's two lowest bits:
+ * its results go to the register in place of the tile. */
+#define DK_FX_STORE 4u
 
 /* One step of a flush plan. */
 typedef struct dk_step {
@@ -240,6 +326,25 @@ int dk_plan_build(const dk_flat_op *ops, int nops, unsigned n, int prec,
 		  const dk_plan_limits *lim, dk_plan *plan);
 void dk_plan_free(dk_plan *plan);
 int dk_gate_classify(const struct dk_gate *g);
+
+/* A wavefront-group shape of a sweep's shared-memory accesses, and the search
+ * for the bank map that serves a list of them (see dk_plan.c). */
+typedef struct dk_bank_pat {
+	int w; /* accesses of this shape per tile */
+	int nb;
+	uint8_t b[4]; /* tile bits varied by the lanes of one wavefront group */
+} dk_bank_pat;
+void dk_choose_bank_map(const dk_bank_pat *pat, int np, int m, int sw, unsigned *F);
+
+/* The planner with factored sweeps (dk_plan_fx.c), one step at a time so that
+ * a sweep can run while the next is planned.  dk_fx_next fills `step` and
+ * *prog (valid until the next call; generic steps have none) and returns 1,
+ * 0 when every gate has been planned, or a negative status. */
+typedef struct dk_fx_plan dk_fx_plan;
+int dk_fx_begin(const dk_flat_op *ops, int nops, unsigned n, int prec,
+		const dk_plan_limits *lim, dk_fx_plan **out);
+int dk_fx_next(dk_fx_plan *p, dk_step *step, const unsigned char **prog);
+void dk_fx_end(dk_fx_plan *p);
 
 /* Debug builds only (libdokigpu_dbg.so, -DDK_DEBUG_CHECKS): the first failed
  * kernel index check since the last reset, 0 if none (site in bits 56-63,

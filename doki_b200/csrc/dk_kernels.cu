@@ -1247,6 +1247,8 @@ __global__ void __launch_bounds__(256, 2)
 	}
 }
 
+#include "dk_sweep_fx.cuh"
+
 enum { FIN_GATE = 0, FIN_COLLAPSE = 1, FIN_RESET = 2 };
 
 /* Sum the (in, out) partials of `nb` blocks in a fixed order and update the
@@ -2438,6 +2440,90 @@ static cudaError_t run_sweep_tm(const void *in, void *out, const unsigned char *
 	*blocks_out = (int)blocks;
 	g_tm_ran.store(1);
 	(pre ? g_tm_presplit : g_tm_entry_b).fetch_add(1, std::memory_order_relaxed);
+	return cudaGetLastError();
+}
+
+/* CTAs of a factored sweep on an SM: what registers allow (128 a thread for
+ * complex128, 80 for complex64); their tiles and programs fit beside each
+ * other (DK_FX_BYTES). */
+template <typename R> struct FxShape;
+template <> struct FxShape<double> {
+	static constexpr int ctas = 2;
+};
+template <> struct FxShape<float> {
+	static constexpr int ctas = 3;
+};
+
+template <typename R>
+static cudaError_t run_sweep_fx(const void *in, void *out, const unsigned char *dprog,
+				const dk_sweep_hdr *hp, int sums, int num_sms, const Scratch &s,
+				cudaStream_t st, int *blocks_out)
+{
+	typedef typename CT<R>::T C2;
+	constexpr int MINB = FxShape<R>::ctas;
+	const size_t smem = (sizeof(C2) << hp->m) + hp->bytes;
+	auto kern = k_sweep_fx<R, MINB>;
+	/* raised once to the device maximum, never lowered (see run_sweep) */
+	static std::once_flag once;
+	static cudaError_t set_err = cudaSuccess;
+	static size_t sm_bytes = 0, cta_bytes = 0; /* of an SM; fixed part of a CTA */
+	std::call_once(once, [&] {
+		int dev = 0, maxopt = 0, maxsm = 0, reserved = 0;
+		cudaGetDevice(&dev);
+		set_err = cudaDeviceGetAttribute(&maxopt, cudaDevAttrMaxSharedMemoryPerBlockOptin,
+						 dev);
+		if (set_err == cudaSuccess)
+			set_err = cudaDeviceGetAttribute(
+				&maxsm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+		if (set_err == cudaSuccess)
+			set_err = cudaDeviceGetAttribute(
+				&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev);
+		cudaFuncAttributes fa;
+		memset(&fa, 0, sizeof(fa));
+		if (set_err == cudaSuccess)
+			set_err = cudaFuncGetAttributes(&fa, kern);
+		if (set_err == cudaSuccess)
+			set_err = cudaFuncSetAttribute(kern,
+						       cudaFuncAttributeMaxDynamicSharedMemorySize,
+						       maxopt - (int)fa.sharedSizeBytes);
+		sm_bytes = (size_t)maxsm;
+		cta_bytes = fa.sharedSizeBytes + (size_t)reserved;
+	});
+	cudaError_t e = set_err;
+	if (e != cudaSuccess)
+		return e;
+	uint64_t per_sm = sm_bytes / (smem + cta_bytes);
+	if (per_sm > MINB)
+		per_sm = MINB;
+	if (per_sm < 1)
+		per_sm = 1;
+	uint64_t blocks = hp->ntiles;
+	if (blocks > per_sm * (uint64_t)num_sms)
+		blocks = per_sm * (uint64_t)num_sms;
+	blocks = skip_balanced_grid(blocks, in, out, hp);
+	kern<<<(int)blocks, 1 << (hp->m - DK_FX_BITS), smem, st>>>((const C2 *)in, (C2 *)out, dprog,
+								     sums, s.partials);
+	*blocks_out = (int)blocks;
+	return cudaGetLastError();
+}
+
+cudaError_t launch_sweep_fx(int prec, const void *in, void *out, const unsigned char *dprog,
+			    const dk_sweep_hdr *hp, int sums, const dk_scal *sc_in, dk_scal *sc_out,
+			    const Scratch &s, int num_sms, cudaStream_t st)
+{
+	g_num_sms = num_sms;
+	int blocks = 0;
+	cudaError_t e = prec == DK_C128
+				? run_sweep_fx<double>(in, out, dprog, hp, sums, num_sms, s, st, &blocks)
+				: run_sweep_fx<float>(in, out, dprog, hp, sums, num_sms, s, st, &blocks);
+	if (e != cudaSuccess)
+		return e;
+	g_launches += 1;
+	if (sums) {
+		const int all = hp->all_touched || (in != out);
+		k_finalize<<<1, 256, 0, st>>>(s.partials, blocks, sc_in, sc_out, FIN_GATE, all);
+		g_launches += 1;
+	}
 	return cudaGetLastError();
 }
 

@@ -47,6 +47,13 @@ cudaError_t launch_sweep(int prec, const void *in, void *out,
 			 const dk_scal *sc_in, dk_scal *sc_out,
 			 const Scratch &s, int num_sms, cudaStream_t st);
 
+/* factored sweep (dk_plan_fx.c); `sums`: also the sums of |amp|^2 and the
+ * output scalars, which only the last sweep of a flush and the one before a
+ * sweep that skips tiles need */
+cudaError_t launch_sweep_fx(int prec, const void *in, void *out, const unsigned char *dprog,
+			    const dk_sweep_hdr *hprog, int sums, const dk_scal *sc_in,
+			    dk_scal *sc_out, const Scratch &s, int num_sms, cudaStream_t st);
+
 /* generic k-qubit gate, out of place */
 cudaError_t launch_generic_gate(int prec, const void *in, void *out,
 				unsigned n, unsigned k, const unsigned *tg,

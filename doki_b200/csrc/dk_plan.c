@@ -665,11 +665,7 @@ typedef struct fold_params {
  * v_b of the bits above SW that minimise the wavefronts of the accesses the
  * sweep's kernel makes, and derives the slot tables from the raw ones. */
 
-typedef struct bank_pat {
-	int w; /* accesses of this shape per tile */
-	int nb;
-	uint8_t b[4]; /* tile bits varied by the lanes of one wavefront group */
-} bank_pat;
+typedef dk_bank_pat bank_pat;
 
 static int gf2_rank(const unsigned *v, int k)
 {
@@ -755,7 +751,7 @@ static int bank_patterns(const dk_pass_desc *pd, int npass, int sw, int mode, ba
 /* Local search for the v_b (b >= sw) of a tile of m bits, starting from the
  * residue map and from a few fixed pseudo-random maps; the cheapest wins
  * (the residue map on ties).  F: m entries, F[b] = e_b for b < sw. */
-static void choose_bank_map(const bank_pat *pat, int np, int m, int sw, unsigned *F)
+void dk_choose_bank_map(const bank_pat *pat, int np, int m, int sw, unsigned *F)
 {
 	const unsigned nv = 1u << sw;
 	unsigned best[16], cur[16];
@@ -1374,7 +1370,7 @@ static int emit_sweep(blob_t *b, const dk_flat_op *ops, const int *idx,
 		if (pat) {
 			unsigned F[16];
 			const int np = bank_patterns(passes, npass, res, mode, pat);
-			choose_bank_map(pat, np, m, res, F);
+			dk_choose_bank_map(pat, np, m, res, F);
 			h->bankv = apply_bank_map(passes, npass, F, m, res);
 			free(pat);
 		} else {

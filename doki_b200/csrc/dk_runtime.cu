@@ -36,7 +36,19 @@ struct Slot {
 	cudaStream_t st = nullptr;
 	dk::Scratch scratch{};
 	std::recursive_mutex mu;
+	/* Sweep programs on their way to the device: a page-locked buffer and a
+	 * device buffer of the same layout, filled in turn in kStageParts parts.
+	 * A part is refilled only after the copies out of it have run (`copied`);
+	 * the device side needs no wait, since copies and sweeps share the
+	 * slot's stream.  Allocated by the slot's first flush, kept with it. */
+	unsigned char *stage_host = nullptr, *stage_dev = nullptr;
+	size_t stage_at = 0;
+	cudaEvent_t copied[2] = { nullptr, nullptr };
+	bool in_use[2] = { false, false };
 };
+
+constexpr size_t kStagePart = 1u << 20;
+constexpr int kStageParts = 2;
 
 constexpr int kMaxSlots = 64;
 
@@ -54,6 +66,8 @@ struct Ctx {
 	int tile_bits = 0; /* 0: planner default */
 	int fold = 0; /* pass-folding cost: 0 planner default, < 0 off */
 	int tensor = 0; /* tensor-core sweeps: 0 planner default (on), < 0 off */
+	/* factored sweeps (dk_plan_fx.c) by precision */
+	int fx_c128 = 1, fx_c64 = 1;
 	int low_bits = -1; /* qubits always in a sweep's tile: < 0 planner default */
 	std::atomic<unsigned long long> sweeps{ 0 }, gates{ 0 }, h2d{ 0 }, d2h{ 0 };
 	/* tensor sweeps: sum of matrix entries x register amplitudes */
@@ -266,6 +280,126 @@ int flush(dk_state *s)
 	}
 }
 
+/* Device copy of `bytes` of host data, valid for work queued on the slot's
+ * stream before the slot's next kStagePart bytes.  The host data may be
+ * reused when the call returns.  Data larger than a part gets an allocation of
+ * its own (*own, freed by the caller after the work that reads it). */
+static int stage_up(const void *src, size_t bytes, const unsigned char **dev, void **own,
+		    size_t *own_bytes)
+{
+	Slot &sl = CUR;
+	*own = nullptr;
+	g.h2d += bytes;
+	if (bytes > kStagePart) {
+		int rc = dev_alloc(own, bytes);
+		if (rc)
+			return rc;
+		*own_bytes = bytes;
+		*dev = (const unsigned char *)*own;
+		/* pageable source: staged before the call returns */
+		cudaError_t e = cudaMemcpyAsync(*own, src, bytes, cudaMemcpyHostToDevice, sl.st);
+		if (e != cudaSuccess) {
+			dev_free(*own, bytes);
+			*own = nullptr;
+			return cuda_fail(e);
+		}
+		return DK_OK;
+	}
+	if (!sl.stage_host) {
+		for (int i = 0; i < kStageParts; ++i)
+			if (!sl.copied[i])
+				CK(cudaEventCreateWithFlags(&sl.copied[i], cudaEventDisableTiming));
+		if (!sl.stage_dev)
+			CK(cudaMalloc(&sl.stage_dev, kStagePart * kStageParts));
+		CK(cudaHostAlloc(&sl.stage_host, kStagePart * kStageParts, cudaHostAllocDefault));
+	}
+	int part = (int)(sl.stage_at / kStagePart);
+	if (sl.stage_at + bytes > (size_t)(part + 1) * kStagePart) {
+		/* the next part: its last copies must have left the host buffer */
+		CK(cudaEventRecord(sl.copied[part], sl.st));
+		sl.in_use[part] = true;
+		part = (part + 1) % kStageParts;
+		sl.stage_at = (size_t)part * kStagePart;
+		if (sl.in_use[part])
+			CK(cudaEventSynchronize(sl.copied[part]));
+	}
+	memcpy(sl.stage_host + sl.stage_at, src, bytes);
+	CK(cudaMemcpyAsync(sl.stage_dev + sl.stage_at, sl.stage_host + sl.stage_at, bytes,
+			   cudaMemcpyHostToDevice, sl.st));
+	*dev = sl.stage_dev + sl.stage_at;
+	sl.stage_at += (bytes + 255) & ~(size_t)255;
+	if (sl.stage_at >= kStagePart * kStageParts)
+		sl.stage_at = kStagePart * kStageParts - 1; /* full: the next call moves on */
+	return DK_OK;
+}
+
+/* Steps of a flush, from either planner. */
+struct StepSource {
+	const std::vector<dk_flat_op> &ops;
+	dk_fx_plan *fx = nullptr;
+	dk_plan plan{};
+	int at = 0;
+	explicit StepSource(const std::vector<dk_flat_op> &o) : ops(o) {}
+	~StepSource()
+	{
+		if (fx)
+			dk_fx_end(fx);
+		dk_plan_free(&plan);
+	}
+	/* 1: a step, 0: none left, < 0: -status */
+	int next(dk_step *step, const unsigned char **prog)
+	{
+		if (fx)
+			return dk_fx_next(fx, step, prog);
+		if (at >= plan.nsteps)
+			return 0;
+		*step = plan.steps[at++];
+		*prog = step->kind == 1 ? plan.blob + step->prog_off : nullptr;
+		return 1;
+	}
+};
+
+/* A planned step whose data is on its way to the device; launched once the
+ * step after it is known. */
+struct ReadyStep {
+	bool have = false;
+	dk_step step{};
+	dk_sweep_hdr hdr{};
+	unsigned long long entries = 0;
+	const unsigned char *dev = nullptr;
+	void *own = nullptr;
+	size_t own_bytes = 0;
+};
+
+static int ready_step(const std::vector<dk_flat_op> &ops, unsigned n, const dk_step &step,
+		      const unsigned char *prog, ReadyStep *r)
+{
+	r->step = step;
+	r->entries = 0;
+	const void *src;
+	size_t bytes;
+	if (step.kind == 1) {
+		memcpy(&r->hdr, prog, sizeof(r->hdr));
+		src = prog;
+		bytes = r->hdr.bytes;
+		if (r->hdr.mode == DK_SWEEP_TENSOR) {
+			const dk_pass_desc *pd = (const dk_pass_desc *)(prog + r->hdr.pass_off);
+			for (int p = 0; p < r->hdr.npass; ++p)
+				r->entries += (unsigned long long)(pd[p].g1 - pd[p].g0);
+		} else if (r->hdr.mode == DK_SWEEP_FACTORED) {
+			r->entries = (unsigned long long)r->hdr.npass;
+		}
+		r->entries <<= n;
+	} else {
+		const dk_gate *gt = ops[step.op_index].gate;
+		src = gt->m;
+		bytes = 16 * gt->dim * gt->dim;
+	}
+	int rc = stage_up(src, bytes, &r->dev, &r->own, &r->own_bytes);
+	r->have = rc == DK_OK;
+	return rc;
+}
+
 static int flush_queued(dk_state *s)
 {
 	DK_TRACE();
@@ -296,84 +430,71 @@ static int flush_queued(dk_state *s)
 	/* complex64 tensor sweeps of 12-bit tiles run on the tcgen05 kernel
 	 * (whole columns per thread) unless DK_C64_TMEM=0 */
 	lim.bank_mode = (prec == DK_C64 && dk::g_c64_tmem) ? 1 : 0;
+	const bool fx = lim.tensor > 0 && g.fuse && lim.tile_bits >= DK_FX_MIN_TILE &&
+			(prec == DK_C64 ? g.fx_c64 : g.fx_c128);
+	/* Factored complex64 sweeps pin 4 low qubits (128-byte runs, as complex128
+	 * sweeps pin 2 for 64-byte ones): at 28 qubits, depth 20, 36 and 34 sweeps
+	 * (brickwork, random pairs) in 59.5 and 56.7 ms against 30 and 29 sweeps in
+	 * 60.4 and 61.3 ms with 2 pinned.  complex128: 107.2 and 107.0 ms with 2,
+	 * 112.6 and 108.0 ms with 4. */
+	if (fx && prec == DK_C64)
+		lim.low_bits = 4;
 	if (g.low_bits >= 0 && g.low_bits <= lim.tile_bits)
 		lim.low_bits = g.low_bits;
-	dk_plan plan;
-	int rc = dk_plan_build(ops.data(), (int)cnt, n, prec, &lim, &plan);
+	StepSource from(ops);
+	int rc = fx ? dk_fx_begin(ops.data(), (int)cnt, n, prec, &lim, &from.fx)
+			 : dk_plan_build(ops.data(), (int)cnt, n, prec, &lim, &from.plan);
 	if (rc)
 		return rc;
-
-	/* device copy of the sweep programs and of generic-gate matrices */
-	size_t gen_bytes = 0;
-	for (int i = 0; i < plan.nsteps; ++i)
-		if (plan.steps[i].kind == 2)
-			gen_bytes += 16 * ops[plan.steps[i].op_index].gate->dim *
-				     ops[plan.steps[i].op_index].gate->dim;
-	const size_t blob_al = (plan.blob_bytes + 255) & ~(size_t)255;
-	unsigned char *dblob = nullptr;
-	rc = dev_alloc((void **)&dblob, blob_al + gen_bytes);
-	if (rc) {
-		dk_plan_free(&plan);
-		return rc;
-	}
-	std::vector<size_t> gen_off(plan.nsteps, 0);
-	{
-		std::vector<unsigned char> host(blob_al + gen_bytes);
-		if (plan.blob_bytes)
-			memcpy(host.data(), plan.blob, plan.blob_bytes);
-		size_t off = blob_al;
-		for (int i = 0; i < plan.nsteps; ++i)
-			if (plan.steps[i].kind == 2) {
-				const dk_gate *gt = ops[plan.steps[i].op_index].gate;
-				memcpy(host.data() + off, gt->m, 16 * gt->dim * gt->dim);
-				gen_off[i] = off;
-				off += 16 * gt->dim * gt->dim;
-			}
-		cudaError_t e = cudaMemcpyAsync(dblob, host.data(), host.size(),
-						cudaMemcpyHostToDevice, CUR.st);
-		if (e != cudaSuccess) {
-			dev_free(dblob, blob_al + gen_bytes);
-			dk_plan_free(&plan);
-			return cuda_fail(e);
-		}
-		/* pageable source: the bytes are staged before the call returns, so
-		 * `host` may be released without waiting for the stream */
-		g.h2d += host.size();
-	}
 
 	dk_buf *src = s->buf;
 	dk_buf *dst = src;
 	if (src->refcount > 1) {
 		rc = buf_new(n, prec, &dst);
-		if (rc) {
-			dev_free(dblob, blob_al + gen_bytes);
-			dk_plan_free(&plan);
+		if (rc)
 			return rc;
-		}
 	}
 	const void *cur = src->d;
 	const dk_scal *cur_sc = src->sc;
-	for (int i = 0; i < plan.nsteps && rc == DK_OK; ++i) {
-		const dk_step &stp = plan.steps[i];
+	ReadyStep ready, next;
+	bool launched = false;
+	dk_step step;
+	const unsigned char *prog = nullptr;
+	/* Each step is launched as soon as the one after it has been planned:
+	 * the device works while the host plans.  The step after it decides
+	 * whether a factored sweep must leave its scalars. */
+	int more = from.next(&step, &prog);
+	if (more > 0)
+		rc = ready_step(ops, n, step, prog, &ready);
+	while (rc == DK_OK && ready.have) {
+		next.have = false;
+		more = from.next(&step, &prog);
+		if (more > 0)
+			rc = ready_step(ops, n, step, prog, &next);
+		else if (more < 0)
+			rc = -more;
+		if (rc)
+			break;
 		cudaError_t e;
-		if (stp.kind == 1) {
-			const dk_sweep_hdr *hp =
-				(const dk_sweep_hdr *)(plan.blob + stp.prog_off);
-			e = dk::launch_sweep(prec, cur, dst->d, dblob + stp.prog_off, hp,
-					     cur_sc, dst->sc, CUR.scratch, g.num_sms, CUR.st);
-			g.sweeps++;
-			if (hp->mode == DK_SWEEP_TENSOR) {
-				const dk_pass_desc *pd = (const dk_pass_desc *)(plan.blob +
-										 stp.prog_off +
-										 hp->pass_off);
-				unsigned long long entries = 0;
-				for (int p = 0; p < hp->npass; ++p)
-					entries += (unsigned long long)(pd[p].g1 - pd[p].g0);
-				g.mma_entry_amps += entries << n;
+		launched = true;
+		if (ready.step.kind == 1) {
+			const dk_sweep_hdr *hp = &ready.hdr;
+			if (hp->mode == DK_SWEEP_FACTORED) {
+				/* the next sweep is in place: it skips tiles, and then
+				 * needs this one's csq, unless it acts on all of them */
+				const int sums = !next.have || (next.step.kind == 1 &&
+								!next.hdr.all_touched);
+				e = dk::launch_sweep_fx(prec, cur, dst->d, ready.dev, hp, sums, cur_sc,
+							dst->sc, CUR.scratch, g.num_sms, CUR.st);
+			} else {
+				e = dk::launch_sweep(prec, cur, dst->d, ready.dev, hp, cur_sc, dst->sc,
+						     CUR.scratch, g.num_sms, CUR.st);
 			}
-			g.gates += (unsigned long long)stp.ngates;
+			g.sweeps++;
+			g.mma_entry_amps += ready.entries;
+			g.gates += (unsigned long long)ready.step.ngates;
 		} else {
-			const dk_flat_op &op = ops[stp.op_index];
+			const dk_flat_op &op = ops[ready.step.op_index];
 			void *target = dst->d;
 			void *tmp = nullptr;
 			if (cur == dst->d) {
@@ -383,8 +504,7 @@ static int flush_queued(dk_state *s)
 				target = tmp;
 			}
 			e = dk::launch_generic_gate(prec, cur, target, n, op.k, op.tg,
-						    op.cm, op.am,
-						    (const double *)(dblob + gen_off[i]),
+						    op.cm, op.am, (const double *)ready.dev,
 						    cur_sc, dst->sc, CUR.scratch, CUR.st);
 			if (tmp) {
 				dev_free(dst->d, dst->bytes);
@@ -396,12 +516,28 @@ static int flush_queued(dk_state *s)
 			rc = cuda_fail(e);
 		cur = dst->d;
 		cur_sc = dst->sc;
+		if (ready.own)
+			dev_free(ready.own, ready.own_bytes);
+		ready = next;
+		next = ReadyStep();
 	}
-	dev_free(dblob, blob_al + gen_bytes);
-	dk_plan_free(&plan);
+	if (rc == DK_OK && more < 0)
+		rc = -more;
+	if (ready.have && ready.own)
+		dev_free(ready.own, ready.own_bytes);
+	if (next.have && next.own)
+		dev_free(next.own, next.own_bytes);
 	if (rc) {
-		if (dst != src)
+		if (dst != src) {
 			buf_release(dst);
+		} else if (launched) {
+			/* some of the gates have already changed the register in
+			 * place: it must not be read, or the rest queued again */
+			op_release(s->pending);
+			s->pending = nullptr;
+			state_drop_caches(s);
+			s->released = 1;
+		}
 		return rc;
 	}
 	if (dst != src) {
@@ -570,9 +706,15 @@ int dk_init(int device)
 	const char *te = getenv("DK_TENSOR");
 	if (te)
 		g.tensor = atoi(te) ? 0 : -1;
+	const char *fx = getenv("DK_FACTORED");
+	if (fx)
+		g.fx_c128 = g.fx_c64 = atoi(fx) ? 1 : 0;
 	const char *tm = getenv("DK_C64_TMEM");
-	if (tm)
+	if (tm) {
+		/* a choice of tensor kernel for complex64 sweeps */
 		dk::g_c64_tmem = atoi(tm) ? 1 : 0;
+		g.fx_c64 = 0;
+	}
 	const char *tp = getenv("DK_C64_TMEM_PRESPLIT");
 	if (tp)
 		dk::g_tm_allow_presplit = atoi(tp) ? 1 : 0;

@@ -191,9 +191,10 @@ int dk_set_fusion(int enable);
  * sweeps executed and gates applied by them.  Any pointer may be NULL. */
 int dk_get_stats(uint64_t *kernel_launches, uint64_t *sweeps,
 		 uint64_t *gates_applied);
-/* Tensor-core sweep work since dk_init: the sum over launched tensor sweeps
- * of (8x8 matrix entries in the sweep) x (amplitudes of the register).  One
- * entry-amplitude is 24 FMA on FP64 MMAs (complex128, Gauss form: 3 real
+/* Fused sweep work since dk_init: the sum over launched sweeps of (products in
+ * the sweep) x (amplitudes of the register).  A product is a pass of a
+ * factored sweep (16 amplitudes of 4 qubits) or an 8x8 matrix entry of a
+ * tensor sweep; one entry-amplitude of the latter is 24 FMA on FP64 MMAs (complex128, Gauss form: 3 real
  * products of 2 m8n8k4 k-steps per 64 amplitudes) or 96 TF32 MMA FMA
  * (complex64: 6 m16n8k8 MMAs per 64 amplitudes). */
 int dk_get_mma_stats(uint64_t *entry_amplitudes);
