@@ -215,6 +215,10 @@ enum { DK_SWEEP_SCALAR = 0, DK_SWEEP_TENSOR = 1, DK_SWEEP_FACTORED = 2 };
  * more sweeps. */
 #define DK_FX_BYTES (40u << 10)
 #define DK_FX_BYTES_SMALL (140u << 10)
+/* Fewest qubits for which a sweep's bank map is searched rather than fixed: the
+ * search takes 10 to 50 us of planning per sweep, more than the bank conflicts
+ * of a small register cost. */
+#define DK_FX_MAP_QUBITS 20
 #define DK_FX_SMALL_TILES 7 /* log2 of the most tiles for a long program */
 
 /* Operation (16 bytes), on the registers a[0..16) of a thread; v is a

@@ -76,6 +76,8 @@ typedef struct fx_gate {
 	int gone; /* absorbed by a later gate */
 	cpx l0, l1, r1;
 	real s, t;
+	cpd d0, d1, dr; /* l0, l1, r1 as the passes use them */
+	double ds, dt;
 } fx_gate;
 
 static uint64_t tbit(unsigned q) { return UINT64_C(1) << q; }
@@ -191,6 +193,8 @@ typedef struct fx_buf {
 	int nlist, clist;
 	dk_gate_cond cond[DK_FX_MAX_CONDS + DK_FX_COND];
 	int ncond;
+	int prec;
+	size_t bytes; /* of the operations and their coefficients in the program */
 	int oom;
 } fx_buf;
 
@@ -236,6 +240,16 @@ static int grow(void **p, size_t elem, int *cap, int want)
 	return 0;
 }
 
+/* Bytes of an operation's coefficients in the program. */
+static size_t op_bytes(const dk_fx_op *o, int prec)
+{
+	if (o->code == DK_FX_STAGE)
+		return 64u + (o->mask & 16u ? (prec == DK_C128 ? 256u : 128u) : 0u);
+	if (o->code < DK_FX_PHASE)
+		return 128;
+	return o->code == DK_FX_PHASE ? 16 : 0;
+}
+
 static dk_fx_op *new_op(fx_buf *b, unsigned code, unsigned mask, uint32_t lc, uint32_t la)
 {
 	if (grow((void **)&b->op, sizeof(dk_fx_op), &b->cop, b->nop + 1)) {
@@ -248,6 +262,7 @@ static dk_fx_op *new_op(fx_buf *b, unsigned code, unsigned mask, uint32_t lc, ui
 	o->coef = (uint32_t)b->ncoef;
 	o->lc = lc;
 	o->la = la;
+	b->bytes += sizeof(*o) + op_bytes(o, b->prec);
 	return o;
 }
 
@@ -272,77 +287,118 @@ static double *new_coef(fx_buf *b, int count)
 
 /* A stage of a pass: diag(din), then rotations along distinct directions,
  * then diag(dout), all in register space.  A stage grows while the next gate's
- * parts commute into it. */
+ * parts commute into it.  Sets of registers are 16-bit masks: M[j] holds the
+ * registers whose pass index has bit j, dinm and doutm those whose factor may
+ * differ from 1 (only these are stored). */
+typedef struct fx_rotn {
+	uint8_t dir, plain; /* plain: along a register bit, co[0] and co[1] for all */
+	double co[16]; /* (x, y) of the 8 pairs */
+} fx_rotn;
+
 typedef struct fx_stage {
 	cpd din[DK_FX_REGS], dout[DK_FX_REGS];
+	uint32_t dinm, doutm, M[DK_FX_BITS];
 	int nrot;
-	uint8_t dir[16];
-	double co[16][16]; /* (x, y) of the 8 pairs */
-	uint8_t L[DK_FX_REGS], Li[DK_FX_REGS]; /* register -> pass index and back */
+	fx_rotn rot[16];
 } fx_stage;
+
+#define ALL16 0xffffu
+static const uint16_t low_regs[DK_FX_BITS] = { 0x5555, 0x3333, 0x0f0f, 0x00ff };
+
+/* The set with every register p replaced by p ^ v. */
+static uint32_t move16(uint32_t m, unsigned v)
+{
+	for (int j = 0; j < DK_FX_BITS; j++)
+		if (v >> j & 1u)
+			m = (m & low_regs[j]) << (1 << j) | (m >> (1 << j) & low_regs[j]);
+	return m;
+}
+
+static unsigned label(const fx_stage *s, unsigned p)
+{
+	unsigned l = 0;
+	for (int j = 0; j < DK_FX_BITS; j++)
+		l |= (s->M[j] >> p & 1u) << j;
+	return l;
+}
+
+/* The register that holds pass index l. */
+static unsigned reg_of(const fx_stage *s, unsigned l)
+{
+	uint32_t m = ALL16;
+	for (int j = 0; j < DK_FX_BITS; j++)
+		m &= l >> j & 1u ? s->M[j] : ~s->M[j];
+	return (unsigned)__builtin_ctz(m);
+}
+
+static unsigned direction(const fx_stage *s, int bit) { return reg_of(s, 0) ^ reg_of(s, 1u << bit); }
 
 /* `cols`: the pass index that register 1 << j holds at the start (linear) */
 static void stage_init(fx_stage *s, const uint8_t *cols)
 {
-	for (unsigned p = 0; p < DK_FX_REGS; p++) {
-		unsigned l = 0;
-		for (int j = 0; j < DK_FX_BITS; j++)
-			if (p >> j & 1u)
-				l ^= cols[j];
-		s->din[p] = s->dout[p] = d_one;
-		s->L[p] = (uint8_t)l;
-		s->Li[l] = (uint8_t)p;
+	for (int j = 0; j < DK_FX_BITS; j++) {
+		s->M[j] = 0;
+		for (int i = 0; i < DK_FX_BITS; i++)
+			if (cols[i] >> j & 1)
+				s->M[j] ^= ALL16 & ~(uint32_t)low_regs[i];
 	}
+	s->dinm = s->doutm = 0;
 	s->nrot = 0;
 }
 
-static void put_diag(fx_buf *b, const cpd *d, int count)
+/* d[p] *= u for the registers of m */
+static void mul_on(cpd *d, uint32_t *dm, uint32_t m, cpd u)
 {
-	double *c = new_coef(b, 2 * count);
-	for (int p = 0; c && p < count; p++) {
-		c[2 * p] = d[p].x;
-		c[2 * p + 1] = d[p].y;
+	if (deq(u, d_one))
+		return;
+	for (uint32_t x = m; x; x &= x - 1) {
+		const int p = __builtin_ctz(x);
+		d[p] = *dm >> p & 1u ? dmul(d[p], u) : u;
+	}
+	*dm |= m;
+}
+
+static void put_diag(fx_buf *b, const cpd *d, uint32_t dm)
+{
+	double *c = new_coef(b, 2 * DK_FX_REGS);
+	for (int p = 0; c && p < DK_FX_REGS; p++) {
+		const cpd v = dm >> p & 1u ? d[p] : d_one;
+		c[2 * p] = v.x;
+		c[2 * p + 1] = v.y;
 	}
 }
 
-/* One value besides 1: the registers that have it in *mask, the value in *u.
- * 0 when there are more. */
-static int single_phase(const cpd *d, unsigned *mask, cpd *u)
+/* A diagonal product (1 outside dm) as one operation; a product of several
+ * values is left to the caller's stage when `full` is given. */
+static void emit_diag(fx_buf *b, const cpd *d, uint32_t dm, uint32_t lc, uint32_t la, int *full)
 {
-	*mask = 0;
-	*u = d_one;
-	for (int p = 0; p < DK_FX_REGS; p++) {
-		if (deq(d[p], d_one))
-			continue;
-		if (!*mask)
-			*u = d[p];
-		else if (!deq(d[p], *u))
-			return 0;
-		*mask |= 1u << p;
-	}
-	return 1;
-}
-
-/* A diagonal product as one operation; a product of several values is left
- * to the caller's stage when `full` is given. */
-static void emit_diag(fx_buf *b, const cpd *d, uint32_t lc, uint32_t la, int *full)
-{
-	cpd u;
-	unsigned mask;
+	cpd u = d_one;
+	uint32_t mask = 0;
+	int one = 1;
 	if (full)
 		*full = 0;
-	if (single_phase(d, &mask, &u)) {
+	for (uint32_t x = dm; x && one; x &= x - 1) {
+		const int p = __builtin_ctz(x);
+		if (deq(d[p], d_one))
+			continue;
 		if (!mask)
-			return;
-		if (u.x == -1 && u.y == 0) {
-			new_op(b, DK_FX_NEG, mask, lc, la);
-			return;
+			u = d[p];
+		one = deq(d[p], u);
+		mask |= 1u << p;
+	}
+	if (one && !mask)
+		return;
+	if (one && u.x == -1 && u.y == 0) {
+		new_op(b, DK_FX_NEG, mask, lc, la);
+		return;
+	}
+	if (one && (popc(mask) <= DK_FX_REGS / 2 || !full)) {
+		double *c;
+		if (new_op(b, DK_FX_PHASE, mask, lc, la) && (c = new_coef(b, 2)) != NULL) {
+			c[0] = u.x;
+			c[1] = u.y;
 		}
-		if (popc(mask) <= DK_FX_REGS / 2 || !full) {
-			if (new_op(b, DK_FX_PHASE, mask, lc, la))
-				put_diag(b, &u, 1);
-			return;
-		}
+		return;
 	}
 	if (full) {
 		*full = 1;
@@ -352,41 +408,33 @@ static void emit_diag(fx_buf *b, const cpd *d, uint32_t lc, uint32_t la, int *fu
 		double *c = new_coef(b, 8);
 		if (c)
 			memset(c, 0, 8 * sizeof(double));
-		put_diag(b, d, DK_FX_REGS);
+		put_diag(b, d, dm);
 	}
 }
 
-/* The coefficients are the same for all pairs, along a register bit. */
-static int plain_rot(unsigned dir, const double *co)
+static void emit_rot(fx_buf *b, const fx_rotn *r, uint32_t lc, uint32_t la)
 {
-	int one = !(dir & (dir - 1u));
-	for (int i = 1; i < 8 && one; i++)
-		one = co[2 * i] == co[0] && co[2 * i + 1] == co[1];
-	return one;
-}
-
-static void emit_rot(fx_buf *b, unsigned dir, const double *co, uint32_t lc, uint32_t la)
-{
-	const int plain = plain_rot(dir, co);
-	if (!new_op(b, plain ? DK_FX_STAGE : DK_FX_ROT + dir, plain ? dir : 0, lc, la))
+	if (!new_op(b, r->plain ? DK_FX_STAGE : DK_FX_ROT + r->dir, r->plain ? r->dir : 0, lc, la))
 		return;
-	double *c = new_coef(b, plain ? 8 : 16);
-	for (int i = 0; c && i < (plain ? 8 : 16); i++)
-		c[i] = !plain ? co[i] : i >> 1 == __builtin_ctz(dir) ? co[i & 1] : 0.0;
+	double *c = new_coef(b, r->plain ? 8 : 16);
+	for (int i = 0; c && i < (r->plain ? 8 : 16); i++)
+		c[i] = !r->plain ? r->co[i] : i >> 1 == __builtin_ctz(r->dir) ? r->co[i & 1] : 0.0;
 }
 
-/* A rotation of direction dir commutes with a plain one along v: what it adds
- * to a register does not depend on that bit. */
-static int passes_plain(unsigned dir, const double *co, unsigned v)
+/* A rotation commutes with a plain one along v: what it adds to a register
+ * does not depend on that bit. */
+static int passes_plain(const fx_rotn *r, unsigned v)
 {
-	const unsigned low = dir & (0u - dir);
+	const unsigned dir = r->dir, low = dir & (0u - dir);
+	if (r->plain)
+		return 1;
 	double c[DK_FX_REGS];
 	int pr = 0;
 	for (unsigned p = 0; p < DK_FX_REGS; p++) {
 		if (p & low)
 			continue;
-		c[p] = co[2 * pr];
-		c[p ^ dir] = co[2 * pr + 1];
+		c[p] = r->co[2 * pr];
+		c[p ^ dir] = r->co[2 * pr + 1];
 		pr++;
 	}
 	for (unsigned p = 0; p < DK_FX_REGS; p++)
@@ -400,14 +448,14 @@ static int passes_plain(unsigned dir, const double *co, unsigned v)
 static void emit_stage(fx_buf *b, const fx_stage *s)
 {
 	int full, first[4] = { -1, -1, -1, -1 }, rest = 0;
-	emit_diag(b, s->din, 0, 0, &full);
+	emit_diag(b, s->din, s->dinm, 0, 0, &full);
 	unsigned mask = full ? 16u : 0u;
 	for (int i = 0; i < s->nrot; i++) {
-		const int j = __builtin_ctz(s->dir[i]);
-		int ahead = plain_rot(s->dir[i], s->co[i]) && first[j] < 0;
+		const int j = __builtin_ctz(s->rot[i].dir);
+		int ahead = s->rot[i].plain && first[j] < 0;
 		for (int k = 0; k < i && ahead; k++)
 			if (rest >> k & 1)
-				ahead = passes_plain(s->dir[k], s->co[k], s->dir[i]);
+				ahead = passes_plain(&s->rot[k], s->rot[i].dir);
 		if (ahead) {
 			first[j] = i;
 			mask |= 1u << j;
@@ -418,13 +466,13 @@ static void emit_stage(fx_buf *b, const fx_stage *s)
 	if (mask && new_op(b, DK_FX_STAGE, mask, 0, 0)) {
 		double *c = new_coef(b, 8);
 		for (int i = 0; c && i < 8; i++)
-			c[i] = first[i >> 1] >= 0 ? s->co[first[i >> 1]][i & 1] : 0.0;
+			c[i] = first[i >> 1] >= 0 ? s->rot[first[i >> 1]].co[i & 1] : 0.0;
 		if (full)
-			put_diag(b, s->din, DK_FX_REGS);
+			put_diag(b, s->din, s->dinm);
 	}
 	for (int i = 0; i < s->nrot; i++)
 		if (rest >> i & 1)
-			emit_rot(b, s->dir[i], s->co[i], 0, 0);
+			emit_rot(b, &s->rot[i], 0, 0);
 }
 
 /* Emit din and the rotations; dout becomes the next stage's din. */
@@ -432,78 +480,86 @@ static void stage_flush(fx_buf *b, fx_stage *s)
 {
 	if (s->nrot) {
 		emit_stage(b, s);
-		memcpy(s->din, s->dout, sizeof(s->din));
 		s->nrot = 0;
-	} else {
-		for (int p = 0; p < DK_FX_REGS; p++)
-			if (!deq(s->dout[p], d_one))
-				s->din[p] = dmul(s->din[p], s->dout[p]);
+		s->dinm = 0;
 	}
-	for (int p = 0; p < DK_FX_REGS; p++)
-		s->dout[p] = d_one;
+	for (uint32_t x = s->doutm; x; x &= x - 1) {
+		const int p = __builtin_ctz(x);
+		s->din[p] = s->dinm >> p & 1u ? dmul(s->din[p], s->dout[p]) : s->dout[p];
+	}
+	s->dinm |= s->doutm;
+	s->doutm = 0;
 }
 
 /* Emit everything pending: the registers hold the amplitudes themselves. */
 static void stage_drain(fx_buf *b, fx_stage *s)
 {
 	stage_flush(b, s);
-	emit_diag(b, s->din, 0, 0, NULL);
-	for (int p = 0; p < DK_FX_REGS; p++)
-		s->din[p] = d_one;
+	emit_diag(b, s->din, s->dinm, 0, 0, NULL);
+	s->dinm = 0;
 }
 
-/* Constant along direction v. */
-static int invariant(const cpd *d, unsigned v)
+/* The set of pairs (by number) of direction v whose registers are in `sel`. */
+static uint32_t pairs_of(uint32_t sel, unsigned v)
 {
-	for (unsigned p = 0; p < DK_FX_REGS; p++)
-		if (!deq(d[p], d[p ^ v]))
-			return 0;
-	return 1;
-}
-
-/* The amplitudes with pass index in `sel` (a 16-bit set of pass indices,
- * closed under bit b) trade places along bit b: a relabelling when that is
- * affine, else an exchange of registers. */
-static void stage_x(fx_buf *b, fx_stage *s, int bit, uint32_t sel, int affine)
-{
-	if (affine) {
-		for (int p = 0; p < DK_FX_REGS; p++)
-			if (sel >> s->L[p] & 1u)
-				s->L[p] ^= (uint8_t)(1u << bit);
-		for (int p = 0; p < DK_FX_REGS; p++)
-			s->Li[s->L[p]] = (uint8_t)p;
-		return;
-	}
-	stage_flush(b, s);
-	const unsigned v = s->Li[1u << bit] ^ s->Li[0], low = v & (0u - v);
+	const unsigned low = v & (0u - v);
 	uint32_t mask = 0;
 	int pr = 0;
 	for (unsigned p = 0; p < DK_FX_REGS; p++) {
 		if (p & low)
 			continue;
-		if (sel >> s->L[p] & 1u) {
-			const cpd t = s->din[p];
-			mask |= 1u << pr;
-			s->din[p] = s->din[p ^ v];
-			s->din[p ^ v] = t;
-		}
+		mask |= (sel >> p & 1u) << pr;
 		pr++;
 	}
-	new_op(b, DK_FX_SWAP + v, mask, 0, 0);
+	return mask;
 }
 
-static void rot_coefs(const fx_stage *s, const fx_gate *g, int bit, uint32_t sel, unsigned v,
-		      double *co)
+/* The registers of `sel` (closed under the direction of bit b) trade places
+ * along it: a relabelling when that is affine, else an exchange. */
+static void stage_x(fx_buf *b, fx_stage *s, int bit, uint32_t sel, int affine)
+{
+	if (affine) {
+		s->M[bit] ^= sel;
+		return;
+	}
+	stage_flush(b, s);
+	const unsigned v = direction(s, bit), low = v & (0u - v);
+	for (unsigned p = 0; p < DK_FX_REGS; p++) {
+		if ((p & low) || !(sel >> p & 1u))
+			continue;
+		const uint32_t i = s->dinm >> p & 1u, j = s->dinm >> (p ^ v) & 1u;
+		const cpd t = s->din[p];
+		s->din[p] = s->din[p ^ v];
+		s->din[p ^ v] = t;
+		s->dinm = (s->dinm & ~(1u << p | 1u << (p ^ v))) | j << p | i << (p ^ v);
+	}
+	new_op(b, DK_FX_SWAP + v, pairs_of(sel, v), 0, 0);
+}
+
+/* The gate's rotation on the registers of `sel`. */
+static void set_rot(fx_rotn *r, const fx_stage *s, const fx_gate *g, int bit, uint32_t sel, unsigned v)
 {
 	const unsigned low = v & (0u - v);
-	const double gs = (double)g->s, gt = (double)g->t;
+	r->dir = (uint8_t)v;
+	r->plain = 0;
+	if (v == low && sel == ALL16) {
+		/* one bit, every register: plain when all pairs have the same of the
+		 * two orders */
+		const uint32_t first = low_regs[__builtin_ctz(v)], hi = s->M[bit] & first;
+		if (hi == 0 || hi == first) {
+			r->plain = 1;
+			r->co[0] = hi ? g->dt : -g->ds;
+			r->co[1] = hi ? -g->ds : g->dt;
+			return;
+		}
+	}
 	int pr = 0;
 	for (unsigned p = 0; p < DK_FX_REGS; p++) {
 		if (p & low)
 			continue;
-		const int on = sel >> s->L[p] & 1u, hi = s->L[p] >> bit & 1;
-		co[2 * pr] = !on ? 0.0 : hi ? gt : -gs;
-		co[2 * pr + 1] = !on ? 0.0 : hi ? -gs : gt;
+		const int on = sel >> p & 1u, hi = s->M[bit] >> p & 1u;
+		r->co[2 * pr] = !on ? 0.0 : hi ? g->dt : -g->ds;
+		r->co[2 * pr + 1] = !on ? 0.0 : hi ? -g->ds : g->dt;
 		pr++;
 	}
 }
@@ -514,120 +570,101 @@ static void rot_coefs(const fx_stage *s, const fx_gate *g, int bit, uint32_t sel
 static void add_gate(fx_buf *b, fx_stage *s, const dk_flat_op *op, const fx_gate *g,
 		     const int *treg, uint32_t cr, uint32_t ar, uint32_t lc, uint32_t la)
 {
-	const cpd l0 = cd(g->l0), l1 = cd(g->l1), r1 = cd(g->r1);
-	uint32_t sel = 0; /* pass indices whose controls hold */
-	for (uint32_t i = 0; i < DK_FX_REGS; i++)
-		if ((i & cr) == cr && !(i & ar))
-			sel |= 1u << i;
-	if (g->kind == FX_DIAG) {
-		const double *m = op->gate->m;
-		const uint64_t dim = op->gate->dim;
-		cpd d[DK_FX_REGS];
-		for (int p = 0; p < DK_FX_REGS; p++) {
-			const unsigned i = s->L[p];
-			uint64_t e = 0;
-			for (unsigned t = 0; t < op->k; t++)
-				e |= (uint64_t)(i >> treg[t] & 1u) << t;
-			if (!(sel >> i & 1u))
-				d[p] = d_one;
-			else if (op->k == 1)
-				d[p] = e ? l1 : l0;
-			else
-				d[p] = (cpd){ m[2 * (e * dim + e)], m[2 * (e * dim + e) + 1] };
-		}
-		if (lc | la) {
-			stage_flush(b, s);
-			emit_diag(b, d, lc, la, NULL);
-			return;
-		}
-		for (int p = 0; p < DK_FX_REGS; p++)
-			if (!deq(d[p], d_one))
-				s->dout[p] = dmul(s->dout[p], d[p]);
-		return;
+	uint32_t sel = ALL16; /* registers whose controls hold */
+	for (int j = 0; j < DK_FX_BITS; j++) {
+		if (cr >> j & 1u)
+			sel &= s->M[j];
+		if (ar >> j & 1u)
+			sel &= ~s->M[j];
 	}
 	const int bit = treg[0];
-	const int affine = popc(cr | ar) <= 1;
-	cpd left[DK_FX_REGS];
+	if (g->kind == FX_DIAG) {
+		cpd d[DK_FX_REGS], *to = s->dout;
+		uint32_t dm = 0, *tom = &s->doutm;
+		if (lc | la) {
+			stage_flush(b, s);
+			to = d;
+			tom = &dm;
+		}
+		if (op->k == 1) {
+			mul_on(to, tom, sel & ~s->M[bit], g->d0);
+			mul_on(to, tom, sel & s->M[bit], g->d1);
+		} else {
+			const double *m = op->gate->m;
+			const uint64_t dim = op->gate->dim;
+			for (uint64_t e = 0; e < dim; e++) {
+				uint32_t on = sel;
+				for (unsigned t = 0; t < op->k; t++)
+					on &= e >> t & 1u ? s->M[treg[t]] : ~s->M[treg[t]];
+				mul_on(to, tom, on,
+				       (cpd){ m[2 * (e * dim + e)], m[2 * (e * dim + e) + 1] });
+			}
+		}
+		if (lc | la)
+			emit_diag(b, d, dm, lc, la, NULL);
+		return;
+	}
 	if (lc | la) {
 		/* per thread: nothing may be left pending along the way */
 		stage_drain(b, s);
-		const unsigned v = s->Li[1u << bit] ^ s->Li[0], low = v & (0u - v);
-		if (g->kind == FX_PERM || g->flip) {
-			uint32_t mask = 0;
-			int pr = 0;
-			for (unsigned p = 0; p < DK_FX_REGS; p++) {
-				if (p & low)
-					continue;
-				if (sel >> s->L[p] & 1u)
-					mask |= 1u << pr;
-				pr++;
-			}
-			new_op(b, DK_FX_SWAP + v, mask, lc, la);
-		}
+		const unsigned v = direction(s, bit);
+		cpd d[DK_FX_REGS];
+		uint32_t dm = 0;
+		if (g->kind == FX_PERM || g->flip)
+			new_op(b, DK_FX_SWAP + v, pairs_of(sel, v), lc, la);
 		if (g->kind == FX_ROT) {
-			cpd right[DK_FX_REGS];
-			for (int p = 0; p < DK_FX_REGS; p++)
-				right[p] = (sel >> s->L[p] & 1u) && (s->L[p] >> bit & 1) ? r1 : d_one;
-			emit_diag(b, right, lc, la, NULL);
-			double co[16];
-			rot_coefs(s, g, bit, sel, v, co);
-			emit_rot(b, v, co, lc, la);
+			fx_rotn r;
+			mul_on(d, &dm, sel & s->M[bit], g->dr);
+			emit_diag(b, d, dm, lc, la, NULL);
+			set_rot(&r, s, g, bit, sel, v);
+			emit_rot(b, &r, lc, la);
+			dm = 0;
 		}
-		for (int p = 0; p < DK_FX_REGS; p++)
-			left[p] = !(sel >> s->L[p] & 1u) ? d_one : (s->L[p] >> bit & 1) ? l1 : l0;
-		emit_diag(b, left, lc, la, NULL);
+		mul_on(d, &dm, sel & ~s->M[bit], g->d0);
+		mul_on(d, &dm, sel & s->M[bit], g->d1);
+		emit_diag(b, d, dm, lc, la, NULL);
 		return;
 	}
 	if (g->kind == FX_PERM || g->flip)
-		stage_x(b, s, bit, sel, affine);
-	for (int p = 0; p < DK_FX_REGS; p++)
-		left[p] = !(sel >> s->L[p] & 1u) ? d_one : (s->L[p] >> bit & 1) ? l1 : l0;
+		stage_x(b, s, bit, sel, popc(cr | ar) <= 1);
+	const uint32_t hi = sel & s->M[bit], lo = sel & ~s->M[bit];
 	if (g->kind == FX_ROT) {
-		const unsigned v = s->Li[1u << bit] ^ s->Li[0];
-		cpd right[DK_FX_REGS];
-		for (int p = 0; p < DK_FX_REGS; p++)
-			right[p] = (sel >> s->L[p] & 1u) && (s->L[p] >> bit & 1) ? r1 : d_one;
+		const unsigned v = direction(s, bit);
 		/* into the open stage when the right factor passes its rotations
 		 * and the rotation its trailing product */
-		int join = s->nrot > 0 && s->nrot < 16 && invariant(s->dout, v);
-		for (int i = 0; join && i < s->nrot; i++)
-			join = invariant(right, s->dir[i]);
+		int join = s->nrot > 0 && s->nrot < 16;
+		if (join && s->doutm) {
+			join = move16(s->doutm, v) == s->doutm;
+			for (uint32_t x = s->doutm; join && x; x &= x - 1) {
+				const int p = __builtin_ctz(x);
+				join = deq(s->dout[p], s->dout[(unsigned)p ^ v]);
+			}
+		}
+		for (int i = 0; join && i < s->nrot && !deq(g->dr, d_one); i++)
+			join = move16(hi, s->rot[i].dir) == hi;
 		if (!join)
 			stage_flush(b, s);
-		for (int p = 0; p < DK_FX_REGS; p++)
-			if (!deq(right[p], d_one))
-				s->din[p] = dmul(s->din[p], right[p]);
-		s->dir[s->nrot] = (uint8_t)v;
-		rot_coefs(s, g, bit, sel, v, s->co[s->nrot]);
-		s->nrot++;
+		mul_on(s->din, &s->dinm, hi, g->dr);
+		set_rot(&s->rot[s->nrot++], s, g, bit, sel, v);
 	}
 	/* a common factor goes in front of the rotations, to the product that
 	 * is there in any case */
-	cpd *d = !(cr | ar) && deq(l0, l1) ? s->din : s->dout;
-	for (int p = 0; p < DK_FX_REGS; p++)
-		if (!deq(left[p], d_one))
-			d[p] = dmul(d[p], left[p]);
+	if (sel == ALL16 && deq(g->d0, g->d1)) {
+		mul_on(s->din, &s->dinm, ALL16, g->d0);
+		return;
+	}
+	mul_on(s->dout, &s->doutm, lo, g->d0);
+	mul_on(s->dout, &s->doutm, hi, g->d1);
 }
 
 /* ---- one sweep ------------------------------------------------------------ */
 
-/* Bytes of an operation's coefficients in the program. */
-static size_t op_bytes(const dk_fx_op *o, int prec)
-{
-	if (o->code == DK_FX_STAGE)
-		return 64u + (o->mask & 16u ? (prec == DK_C128 ? 256u : 128u) : 0u);
-	if (o->code < DK_FX_PHASE)
-		return 128;
-	return o->code == DK_FX_PHASE ? 16 : 0;
-}
-
-static size_t coef_bytes(const fx_buf *b, int prec)
-{
-	size_t bytes = 0;
-	for (int i = 0; i < b->nop; i++)
-		bytes += op_bytes(&b->op[i], prec);
-	return bytes;
-}
+/* A gate of a pass. */
+typedef struct listed {
+	int id, cond; /* its tile condition among the pass's, -1: none */
+	int treg[DK_SWEEP_MAX_K];
+	uint32_t cr, ar, lc, la;
+} listed;
 
 /* At most DK_FX_COND past the program's limit, which the caller checks. */
 static int find_cond(fx_buf *b, uint64_t gc, uint64_t ga)
@@ -640,36 +677,37 @@ static int find_cond(fx_buf *b, uint64_t gc, uint64_t ga)
 	return b->ncond++;
 }
 
+/* tile bits of residue r mod sw, sw = 3 and 4 */
+static const uint16_t residue[2][4] = { { 0x9249, 0x2492, 0x4924, 0 },
+					{ 0x1111, 0x2222, 0x4444, 0x8888 } };
+
 /* Thread bits of a pass: lanes first, the low ones on tile bits of distinct
  * residues mod sw where there are such, then the phase's warp bits. */
-static int lane_order(uint32_t L, uint32_t W, int m, int sw, uint8_t *lane)
+static int lane_order(uint32_t L, uint32_t W, int sw, uint8_t *lane)
 {
 	int nl = 0;
 	uint32_t left = L;
-	for (int r = 0; r < sw; r++)
-		for (int b = 0; b < m; b++)
-			if ((left >> b & 1u) && b % sw == r) {
-				lane[nl++] = (uint8_t)b;
-				left &= ~(1u << b);
-				break;
-			}
+	for (int r = 0; r < sw; r++) {
+		const uint32_t x = left & residue[sw - 3][r];
+		if (x) {
+			lane[nl++] = (uint8_t)__builtin_ctz(x);
+			left &= ~(x & (0u - x));
+		}
+	}
 	const int distinct = nl;
-	for (int b = 0; b < m; b++)
-		if (left >> b & 1u)
-			lane[nl++] = (uint8_t)b;
-	for (int b = 0; b < m; b++)
-		if (W >> b & 1u)
-			lane[nl++] = (uint8_t)b;
+	for (; left; left &= left - 1)
+		lane[nl++] = (uint8_t)__builtin_ctz(left);
+	for (; W; W &= W - 1)
+		lane[nl++] = (uint8_t)__builtin_ctz(W);
 	return distinct;
 }
 
-static int residues(uint32_t L, int m, int sw)
+static int residues(uint32_t L, int sw)
 {
-	unsigned seen = 0;
-	for (int b = 0; b < m; b++)
-		if (L >> b & 1u)
-			seen |= 1u << (b % sw);
-	return popc(seen);
+	int n = 0;
+	for (int r = 0; r < sw; r++)
+		n += (L & residue[sw - 3][r]) != 0;
+	return n;
 }
 
 /* Passes [p0, p1), whose target bits fit in m - wbits tile bits: complete
@@ -697,16 +735,14 @@ static void lay_out_phase(dk_fx_plan *P, int p0, int p1, int m, int wbits, int s
 		pool &= ~3u;
 	uint32_t W = 0;
 	int best = -1;
-	for (uint32_t x = pool;; x = (x - 1) & pool) {
+	for (uint32_t x = pool; best < sw * (p1 - p0); x = (x - 1) & pool) {
 		if (popc(x) == wbits) {
 			int sc = 0;
 			for (int i = p0; i < p1; i++)
-				sc += residues(all & ~P->need[i] & ~x, m, sw);
+				sc += residues(all & ~P->need[i] & ~x, sw);
 			if (sc > best) {
 				best = sc;
 				W = x;
-				if (sc == sw * (p1 - p0))
-					break;
 			}
 		}
 		if (x == 0)
@@ -719,7 +755,7 @@ static void lay_out_phase(dk_fx_plan *P, int p0, int p1, int m, int wbits, int s
 		for (int b = 0; b < m; b++)
 			if (B >> b & 1u)
 				P->pbits[i][j++] = (uint8_t)b;
-		if (lane_order(all & ~B & ~W, W, m, sw, lanes[i]) < sw)
+		if (lane_order(all & ~B & ~W, W, sw, lanes[i]) < sw)
 			*conflicts = 1;
 		if (i + 1 < p1)
 			pd->flags |= DK_PASS_WARP;
@@ -911,7 +947,7 @@ static int emit(dk_fx_plan *P, int cnt, uint64_t Q, int m, dk_step *step,
 	unsigned F[16];
 	for (int b = 0; b < m; b++)
 		F[b] = 1u << (b % sw);
-	if (conflicts) {
+	if (conflicts && n >= DK_FX_MAP_QUBITS) {
 		/* some pass has no lanes on sw distinct residues: search a map */
 		dk_bank_pat pat[DK_MAX_FX_PASSES];
 		for (int i = 0; i < npass; i++) {
@@ -929,24 +965,44 @@ static int emit(dk_fx_plan *P, int cnt, uint64_t Q, int m, dk_step *step,
 	/* operation lists, pass by pass while the program has room */
 	fx_buf *b = &P->b;
 	b->nop = b->nlist = b->ncond = b->oom = 0;
+	b->bytes = 0;
+	b->prec = P->prec;
 	b->ncoef = 0;
 	int all_touched = 0, done = 0;
 	const size_t cap = n <= (unsigned)m + DK_FX_SMALL_TILES ? DK_FX_BYTES_SMALL : DK_FX_BYTES;
 	for (int i = 0; i < npass; i++) {
 		dk_fx_pass *pd = &P->pass[i];
 		const int nop0 = b->nop, nlist0 = b->nlist, ncond0 = b->ncond;
-		const size_t ncoef0 = b->ncoef;
+		const size_t ncoef0 = b->ncoef, bytes0 = b->bytes;
 		int preg[16], touched = 0;
 		memset(preg, -1, sizeof(preg));
 		for (int r = 0; r < DK_FX_BITS; r++)
 			preg[P->pbits[i][r]] = r;
 		/* the pass's conditions */
 		uint64_t gcs[DK_FX_COND], gas[DK_FX_COND];
-		int nc = 0;
+		int nc = 0, np = 0;
+		listed pg[FX_WINDOW]; /* its gates, with their register bits */
 		pd->cond = 0;
 		pd->list = (uint32_t)b->nlist;
 		for (int k = P->range[i][0]; k < P->range[i][1]; k++) {
-			const dk_flat_op *op = &P->ops[P->order[k]];
+			const int id = P->order[k];
+			const dk_flat_op *op = &P->ops[id];
+			listed *e = &pg[np++];
+			memset(e, 0, sizeof(*e));
+			e->id = id;
+			e->cond = -1;
+			for (unsigned t = 0; t < op->k; t++)
+				e->treg[t] = preg[loc[op->tg[t]]];
+			for (uint64_t x = P->g[id].ctl & Q; x; x &= x - 1) {
+				const int q = __builtin_ctzll(x), l = loc[q];
+				const int anti = op->am >> q & 1u;
+				if (preg[l] >= 0)
+					*(anti ? &e->ar : &e->cr) |= 1u << preg[l];
+				else
+					*(anti ? &e->la : &e->lc) |= 1u << l;
+			}
+			if (e->lc | e->la)
+				pd->flags |= DK_PASS_CTL;
 			const uint64_t gc = op->cm & ~Q, ga = op->am & ~Q;
 			int c = 0;
 			if (!(gc | ga)) {
@@ -960,56 +1016,29 @@ static int emit(dk_fx_plan *P, int cnt, uint64_t Q, int m, dk_step *step,
 				gas[nc] = ga;
 				pd->cond |= (uint32_t)find_cond(b, gc, ga) << (5 * nc++);
 			}
+			e->cond = c;
 		}
 		pd->cond |= (uint32_t)nc << 15;
 		if (grow((void **)&b->list, sizeof(dk_fx_list), &b->clist, b->nlist + (1 << nc)))
 			return DK_ERR_ALLOC;
 		for (int v = 0; v < 1 << nc; v++) {
 			dk_fx_list *li = &b->list[b->nlist++];
-			/* the list's gates, with their register bits */
-			typedef struct listed {
-				int id, treg[DK_SWEEP_MAX_K];
-				uint32_t cr, ar, lc, la;
-			} listed;
-			listed gl[FX_WINDOW];
+			const listed *gl[FX_WINDOW];
 			int ng = 0;
-			for (int k = P->range[i][0]; k < P->range[i][1]; k++) {
-				const int id = P->order[k];
-				const dk_flat_op *op = &P->ops[id];
-				const uint64_t gc = op->cm & ~Q, ga = op->am & ~Q;
-				int on = 1;
-				for (int c = 0; c < nc; c++)
-					if (gcs[c] == gc && gas[c] == ga)
-						on = v >> c & 1;
-				if (!on)
-					continue;
-				listed *e = &gl[ng++];
-				memset(e, 0, sizeof(*e));
-				e->id = id;
-				for (unsigned t = 0; t < op->k; t++)
-					e->treg[t] = preg[loc[op->tg[t]]];
-				for (uint64_t x = P->g[id].ctl & Q; x; x &= x - 1) {
-					const int q = __builtin_ctzll(x), l = loc[q];
-					const int anti = op->am >> q & 1u;
-					if (preg[l] >= 0)
-						*(anti ? &e->ar : &e->cr) |= 1u << preg[l];
-					else
-						*(anti ? &e->la : &e->lc) |= 1u << l;
-				}
-				if (e->lc | e->la)
-					pd->flags |= DK_PASS_CTL;
-			}
+			for (int k = 0; k < np; k++)
+				if (pg[k].cond < 0 || (v >> pg[k].cond & 1))
+					gl[ng++] = &pg[k];
 			/* CNOTs relabel the registers: the gather starts from the labels
 			 * under which the most rotations run along a register bit.  rows:
 			 * the linear part of register -> pass index so far, by rows */
 			uint8_t rows[DK_FX_BITS], best[DK_FX_BITS], cols[DK_FX_BITS];
 			for (int j = 0; j < DK_FX_BITS; j++)
-				rows[j] = best[j] = (uint8_t)(1u << j);
-			int cnt = 0, most = 0;
+				rows[j] = best[j] = cols[j] = (uint8_t)(1u << j);
+			int cnt = 0, most = 0, moved = 0;
 			for (int k = 0; k < ng; k++) {
-				const fx_gate *g = &P->g[gl[k].id];
-				const uint32_t c = gl[k].cr | gl[k].ar;
-				if (gl[k].lc | gl[k].la)
+				const fx_gate *g = &P->g[gl[k]->id];
+				const uint32_t c = gl[k]->cr | gl[k]->ar;
+				if (gl[k]->lc | gl[k]->la)
 					continue;
 				if ((g->kind == FX_PERM || (g->kind == FX_ROT && g->flip)) && popc(c) == 1) {
 					if (cnt > most) {
@@ -1017,13 +1046,15 @@ static int emit(dk_fx_plan *P, int cnt, uint64_t Q, int m, dk_step *step,
 						memcpy(best, rows, sizeof(best));
 					}
 					cnt = 0;
-					rows[gl[k].treg[0]] ^= rows[__builtin_ctz(c)];
+					rows[gl[k]->treg[0]] ^= rows[__builtin_ctz(c)];
+					moved = 1;
 				}
 				cnt += g->kind == FX_ROT;
 			}
 			if (cnt > most)
 				memcpy(best, rows, sizeof(best));
-			invert4(best, cols);
+			if (moved)
+				invert4(best, cols);
 			fx_stage s;
 			stage_init(&s, cols);
 			uint32_t gt[DK_FX_BITS];
@@ -1036,35 +1067,31 @@ static int emit(dk_fx_plan *P, int cnt, uint64_t Q, int m, dk_step *step,
 			li->gc = 0;
 			li->op0 = (uint16_t)b->nop;
 			for (int k = 0; k < ng; k++)
-				add_gate(b, &s, &P->ops[gl[k].id], &P->g[gl[k].id], gl[k].treg, gl[k].cr,
-					 gl[k].ar, gl[k].lc, gl[k].la);
+				add_gate(b, &s, &P->ops[gl[k]->id], &P->g[gl[k]->id], gl[k]->treg,
+					 gl[k]->cr, gl[k]->ar, gl[k]->lc, gl[k]->la);
 			stage_drain(b, &s);
-			uint32_t st[DK_FX_BITS];
-			uint32_t full[DK_FX_REGS];
-			for (uint32_t r = 0; r < DK_FX_REGS; r++) {
-				full[r] = 0;
-				for (int j = 0; j < DK_FX_BITS; j++)
-					if (s.L[r] >> j & 1)
-						full[r] ^= P->sp[i][j];
-			}
-			int same = full[0] == 0;
+			unsigned l0 = label(&s, 0), same = l0 == 0;
+			li->lmap = (uint32_t)l0 << 16;
+			li->sc = 0;
 			for (int j = 0; j < DK_FX_BITS; j++) {
-				st[j] = full[1u << j] ^ full[0];
-				same &= st[j] == gt[j];
-			}
-			li->sc = (uint16_t)full[0];
-			li->lmap = (uint32_t)s.L[0] << 16;
-			for (int j = 0; j < DK_FX_BITS; j++) {
+				const unsigned lj = label(&s, 1u << j) ^ l0;
+				uint32_t st = 0;
+				for (int x = 0; x < DK_FX_BITS; x++) {
+					if (lj >> x & 1u)
+						st ^= P->sp[i][x];
+				}
+				if (l0 >> j & 1u)
+					li->sc ^= (uint16_t)P->sp[i][j];
+				same &= st == gt[j];
 				li->gt[j] = (uint16_t)gt[j];
-				li->st[j] = (uint16_t)st[j];
-				li->lmap |= (uint32_t)(s.L[1u << j] ^ s.L[0]) << (4 * j);
+				li->st[j] = (uint16_t)st;
+				li->lmap |= (uint32_t)lj << (4 * j);
 			}
 			li->op1 = (uint16_t)b->nop;
 			li->idle = same && li->op0 == li->op1;
 		}
 		const size_t bytes = sizeof(dk_sweep_hdr) + sizeof(dk_fx_pass) * (size_t)(i + 1) +
-				     sizeof(dk_fx_list) * (size_t)b->nlist +
-				     sizeof(dk_fx_op) * (size_t)b->nop + coef_bytes(b, P->prec) +
+				     sizeof(dk_fx_list) * (size_t)b->nlist + b->bytes +
 				     sizeof(dk_gate_cond) * (size_t)b->ncond;
 		if (b->oom)
 			return DK_ERR_ALLOC;
@@ -1073,6 +1100,7 @@ static int emit(dk_fx_plan *P, int cnt, uint64_t Q, int m, dk_step *step,
 			b->nlist = nlist0;
 			b->ncond = ncond0;
 			b->ncoef = ncoef0;
+			b->bytes = bytes0;
 			const int k0 = P->range[i][0], k1 = P->range[i][1];
 			if (i > 0 || k1 - k0 == 1)
 				break; /* the other gates make another program */
@@ -1107,7 +1135,7 @@ static int emit(dk_fx_plan *P, int cnt, uint64_t Q, int m, dk_step *step,
 	const size_t gate_off = list_off + sizeof(dk_fx_list) * (size_t)b->nlist;
 	const size_t cond_off = gate_off + sizeof(dk_fx_op) * (size_t)b->nop;
 	const size_t mat_off = align16(cond_off + sizeof(dk_gate_cond) * (size_t)b->ncond);
-	const size_t bytes = align16(mat_off + coef_bytes(b, P->prec));
+	const size_t bytes = align16(mat_off + b->bytes - sizeof(dk_fx_op) * (size_t)b->nop);
 	if (bytes > P->cprog) {
 		unsigned char *np = (unsigned char *)realloc(P->prog, 2 * bytes);
 		if (!np)
@@ -1294,7 +1322,7 @@ int dk_fx_begin(const dk_flat_op *ops, int nops, unsigned n, int prec,
 	P->lim = *lim;
 	P->cpass = DK_MAX_FX_PASSES;
 	const size_t cnt = (size_t)(nops > 0 ? nops : 1);
-	P->g = (fx_gate *)malloc(sizeof(fx_gate) * cnt);
+	P->g = (fx_gate *)calloc(cnt, sizeof(fx_gate));
 	P->rem = (int *)malloc(sizeof(int) * cnt);
 	P->take = (int *)malloc(sizeof(int) * cnt);
 	P->order = (int *)malloc(sizeof(int) * cnt);
@@ -1319,6 +1347,12 @@ int dk_fx_begin(const dk_flat_op *ops, int nops, unsigned n, int prec,
 		move_factors(P);
 	P->nops = 0;
 	for (int i = 0; i < nops; i++) {
+		fx_gate *g = &P->g[i];
+		g->d0 = cd(g->l0);
+		g->d1 = cd(g->l1);
+		g->dr = cd(g->r1);
+		g->ds = (double)g->s;
+		g->dt = (double)g->t;
 		if (P->g[i].gone)
 			P->ngone++;
 		else

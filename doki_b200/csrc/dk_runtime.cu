@@ -436,8 +436,9 @@ static int flush_queued(dk_state *s)
 	 * sweeps pin 2 for 64-byte ones): at 28 qubits, depth 20, 36 and 34 sweeps
 	 * (brickwork, random pairs) in 59.5 and 56.7 ms against 30 and 29 sweeps in
 	 * 60.4 and 61.3 ms with 2 pinned.  complex128: 107.2 and 107.0 ms with 2,
-	 * 112.6 and 108.0 ms with 4. */
-	if (fx && prec == DK_C64)
+	 * 112.6 and 108.0 ms with 4.  A register that stays in the L2 cache (below
+	 * 24 qubits) gains nothing from longer runs. */
+	if (fx && prec == DK_C64 && n >= 24)
 		lim.low_bits = 4;
 	if (g.low_bits >= 0 && g.low_bits <= lim.tile_bits)
 		lim.low_bits = g.low_bits;
