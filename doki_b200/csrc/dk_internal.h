@@ -206,7 +206,7 @@ enum { DK_SWEEP_SCALAR = 0, DK_SWEEP_TENSOR = 1, DK_SWEEP_FACTORED = 2 };
 #define DK_FX_BITS 4
 #define DK_FX_REGS 16
 #define DK_FX_COND 3 /* most tile conditions of a pass */
-#define DK_FX_MIN_TILE 9 /* tile bits: a full warp of 16-amplitude columns */
+#define DK_FX_MIN_TILE 4 /* tile bits: one thread's 16 amplitudes */
 #define DK_FX_MAX_GATES 512 /* gates of a sweep */
 #define DK_MAX_FX_PASSES DK_FX_MAX_GATES
 /* Most bytes of a factored program, which the kernel keeps in shared memory:

@@ -2454,7 +2454,7 @@ template <> struct FxShape<float> {
 	static constexpr int ctas = 3;
 };
 
-template <typename R>
+template <typename R, bool NARROW>
 static cudaError_t run_sweep_fx(const void *in, void *out, const unsigned char *dprog,
 				const dk_sweep_hdr *hp, int sums, int num_sms, const Scratch &s,
 				cudaStream_t st, int *blocks_out)
@@ -2462,7 +2462,7 @@ static cudaError_t run_sweep_fx(const void *in, void *out, const unsigned char *
 	typedef typename CT<R>::T C2;
 	constexpr int MINB = FxShape<R>::ctas;
 	const size_t smem = (sizeof(C2) << hp->m) + hp->bytes;
-	auto kern = k_sweep_fx<R, MINB>;
+	auto kern = k_sweep_fx<R, MINB, NARROW>;
 	/* raised once to the device maximum, never lowered (see run_sweep) */
 	static std::once_flag once;
 	static cudaError_t set_err = cudaSuccess;
@@ -2501,8 +2501,9 @@ static cudaError_t run_sweep_fx(const void *in, void *out, const unsigned char *
 	if (blocks > per_sm * (uint64_t)num_sms)
 		blocks = per_sm * (uint64_t)num_sms;
 	blocks = skip_balanced_grid(blocks, in, out, hp);
-	kern<<<(int)blocks, 1 << (hp->m - DK_FX_BITS), smem, st>>>((const C2 *)in, (C2 *)out, dprog,
-								     sums, s.partials);
+	const int threads = NARROW ? 32 : 1 << (hp->m - DK_FX_BITS);
+	kern<<<(int)blocks, threads, smem, st>>>((const C2 *)in, (C2 *)out, dprog, sums,
+						 s.partials);
 	*blocks_out = (int)blocks;
 	return cudaGetLastError();
 }
@@ -2513,9 +2514,16 @@ cudaError_t launch_sweep_fx(int prec, const void *in, void *out, const unsigned 
 {
 	g_num_sms = num_sms;
 	int blocks = 0;
-	cudaError_t e = prec == DK_C128
-				? run_sweep_fx<double>(in, out, dprog, hp, sums, num_sms, s, st, &blocks)
-				: run_sweep_fx<float>(in, out, dprog, hp, sums, num_sms, s, st, &blocks);
+	const bool narrow = hp->m < DK_FX_BITS + 5;
+	cudaError_t e;
+	if (prec == DK_C128)
+		e = narrow ? run_sweep_fx<double, true>(in, out, dprog, hp, sums, num_sms, s, st, &blocks)
+			   : run_sweep_fx<double, false>(in, out, dprog, hp, sums, num_sms, s, st,
+							 &blocks);
+	else
+		e = narrow ? run_sweep_fx<float, true>(in, out, dprog, hp, sums, num_sms, s, st, &blocks)
+			   : run_sweep_fx<float, false>(in, out, dprog, hp, sums, num_sms, s, st,
+							&blocks);
 	if (e != cudaSuccess)
 		return e;
 	g_launches += 1;

@@ -933,7 +933,7 @@ static int emit(dk_fx_plan *P, int cnt, uint64_t Q, int m, dk_step *step,
 		npass++;
 	}
 	/* phases: passes that keep their warp bits need a warp barrier only */
-	const int wbits = m - DK_FX_BITS - 5;
+	const int wbits = m > DK_FX_BITS + 5 ? m - DK_FX_BITS - 5 : 0;
 	uint8_t lanes[DK_MAX_FX_PASSES][16];
 	int conflicts = 0;
 	for (int p0 = 0; p0 < npass;) {

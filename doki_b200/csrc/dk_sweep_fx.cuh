@@ -212,7 +212,7 @@ __device__ __forceinline__ void fx_op(C2 (&a)[DK_FX_REGS], uint32_t code, uint32
 	}
 }
 
-template <typename R, int MINB>
+template <typename R, int MINB, bool NARROW>
 __global__ void __launch_bounds__(256, MINB)
 	k_sweep_fx(const typename CT<R>::T *__restrict__ in, typename CT<R>::T *out,
 		   const unsigned char *__restrict__ prog, int sums, double *partials)
@@ -227,6 +227,9 @@ __global__ void __launch_bounds__(256, MINB)
 	const dk_sweep_hdr *gh = reinterpret_cast<const dk_sweep_hdr *>(prog);
 	const int m = gh->m;
 	const int lanes = m - DK_FX_BITS;
+	/* NARROW: a tile below 9 bits does not fill a warp; its other threads
+	 * follow along on the slots of the first ones and write nothing */
+	const bool writes = !NARROW || tid < (1u << lanes);
 	[[maybe_unused]] const uint32_t tile_bytes = (uint32_t)sizeof(C2) << m;
 	unsigned char *const sp = sm + (sizeof(C2) << m);
 	{
@@ -276,7 +279,7 @@ __global__ void __launch_bounds__(256, MINB)
 		if (!store)
 			off_out = off_t;
 	}
-	const uint32_t stid = (uint32_t)sizeof(C2) * swz_map(tid, h->bankv);
+	const uint32_t stid = (uint32_t)sizeof(C2) * swz_map(tid & ((1u << lanes) - 1u), h->bankv);
 	__syncthreads();
 	const uint64_t ntiles = h->ntiles;
 	const int ndep = (h->n - m + 3) >> 2;
@@ -329,7 +332,7 @@ __global__ void __launch_bounds__(256, MINB)
 		for (int r = 0; r < DK_FX_REGS; ++r) {
 			const uint32_t so = stid ^ bits4(r, s0, s1, s2, s3);
 			const uint64_t gi = at ^ off4(r, o0, o1, o2, o3);
-			if (!DK_IN_BOUNDS(so, tile_bytes, CHK_LOAD_SMEM) ||
+			if (!writes || !DK_IN_BOUNDS(so, tile_bytes, CHK_LOAD_SMEM) ||
 			    !DK_IN_BOUNDS(gi, nglob, CHK_LOAD_GLOBAL))
 				continue;
 			if (sizeof(C2) == 16)
@@ -362,9 +365,10 @@ __global__ void __launch_bounds__(256, MINB)
 		if (skip_idle && sums) {
 			/* only touched tiles reach here: their old |amp|^2 leaves csq */
 			read16(stid, sro[0], sro[1], sro[2], sro[3]);
+			if (writes)
 #pragma unroll
-			for (int r = 0; r < DK_FX_REGS; ++r)
-				insq += sqabs(a[r]);
+				for (int r = 0; r < DK_FX_REGS; ++r)
+					insq += sqabs(a[r]);
 			__syncthreads();
 		}
 		uint64_t g0 = 0, g1 = 0, g2 = 0, g3 = 0, at = cbase * sizeof(C2) ^ off_out;
@@ -426,7 +430,7 @@ __global__ void __launch_bounds__(256, MINB)
 #pragma unroll
 				for (int r = 0; r < DK_FX_REGS; ++r) {
 					const uint32_t x = sc ^ bits4(r, u0, u1, u2, u3);
-					if (DK_IN_BOUNDS(x, tile_bytes, CHK_SCATTER))
+					if (writes && DK_IN_BOUNDS(x, tile_bytes, CHK_SCATTER))
 						*reinterpret_cast<C2 *>(sm + x) = a[r];
 				}
 			}
@@ -447,7 +451,7 @@ __global__ void __launch_bounds__(256, MINB)
 			g2 = soff[2];
 			g3 = soff[3];
 		}
-		if (sums) {
+		if (sums && writes) {
 #pragma unroll
 			for (int r = 0; r < DK_FX_REGS; ++r)
 				outsq += sqabs(a[r]);
@@ -455,7 +459,7 @@ __global__ void __launch_bounds__(256, MINB)
 #pragma unroll
 		for (int r = 0; r < DK_FX_REGS; ++r) {
 			const uint64_t gi = at ^ off4(r, g0, g1, g2, g3);
-			if (DK_IN_BOUNDS(gi, nglob, CHK_STORE))
+			if (writes && DK_IN_BOUNDS(gi, nglob, CHK_STORE))
 				__stcs(reinterpret_cast<C2 *>(reinterpret_cast<unsigned char *>(out) + gi),
 				       a[r]);
 		}

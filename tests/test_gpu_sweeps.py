@@ -26,7 +26,7 @@ def check(d, orc, n, prec, ops, seed):
 
 
 @pytest.mark.parametrize("prec", [2, 1])
-@pytest.mark.parametrize("n", [8, 9, 10, 11, 12, 13, 15, 17])
+@pytest.mark.parametrize("n", [4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 15, 17])
 def test_gates_with_controls_everywhere(dk_gpu, orc, n, prec):
     check(dk_gpu, orc, n, prec, one_qubit_ops(W.rng_for(300 + n), n, 100), 310 + n)
 
