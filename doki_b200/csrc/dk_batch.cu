@@ -1,18 +1,19 @@
 /*
  * Batching form: thousands of independent registers (4-16 qubits), each with
- * its own gate sequence, executed by one persistent kernel per size class,
- * all captured in one CUDA graph.
+ * its own gate sequence, one kernel per size class, all captured in one CUDA
+ * graph.
  *
- * Every circuit is planned with the same planner as the plain path
- * (dk_plan.c): a register of n <= 12 qubits is one tile, so its whole program
- * runs on a shared-memory copy of the register (zero HBM traffic besides the
- * program and the results); a register of 13-16 qubits is owned by one thread
- * group that streams it through tiles of `tile_bits` qubits, sweep after sweep,
- * in a device buffer that stays L2-resident.  A thread group of 2^(m-3)
- * threads owns one register at a time (m = tile bits), several groups share a
- * 512-thread CTA and synchronise with their own barriers.  After the circuit
- * the group computes the register's reduced density matrix over its lower
- * `keep` qubits, renormalised by the trace as the reference's lazy norm does.
+ * Every circuit is planned as in the plain path.  Circuits whose gates all have
+ * a factoring (dk_plan_fx.c) run as factored sweeps: a register of n <= 12
+ * qubits is one tile, owned by 2^(n - 4) threads of a 256-thread CTA that hold it
+ * in shared memory from the first gate to the results (k_batch_fx); a register
+ * of 13-16 qubits is owned by a thread-block cluster whose CTAs share the tiles of
+ * every sweep, with a cluster barrier in between, over a buffer that stays in the
+ * L2 cache (k_batch_cluster).  Circuits with dense 2-qubit gates are planned by
+ * dk_plan.c and run gate by gate on groups of 2^(m - 3) threads (k_batch).
+ * After the circuit the owner computes the register's reduced density matrix
+ * over its lower `keep` qubits, renormalised by the trace as the reference's
+ * lazy norm does.
  */
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -45,6 +46,8 @@ typedef struct dk_breg {
 
 namespace dk {
 namespace {
+
+#include "dk_sweep_fx.cuh"
 
 constexpr int kBatchThreads = 512;
 
@@ -231,6 +234,235 @@ __global__ void __launch_bounds__(kBatchThreads, 1)
 	}
 }
 
+/* ---- factored circuits ---------------------------------------------------- */
+
+constexpr int kFxThreads = 256;
+
+/* Barrier over one register's G threads: the first lanes of a warp, or whole
+ * warps (group gid of a CTA). */
+__device__ __forceinline__ void fx_group_sync(int G, int gid)
+{
+	if (G >= 64)
+		asm volatile("barrier.sync %0, %1;\n" ::"r"(gid + 1), "r"(G) : "memory");
+	else
+		__syncwarp(G >= 32 ? 0xffffffffu : (1u << G) - 1u);
+}
+
+/* Sum over the group's G threads, in a fixed order, in all of them.  r: one
+ * double per thread. */
+__device__ __forceinline__ double fx_group_sum(double v, int G, int gid, uint32_t lt, double *r)
+{
+	r[lt] = v;
+	fx_group_sync(G, gid);
+	for (int st = G >> 1; st > 0; st >>= 1) {
+		if ((int)lt < st)
+			r[lt] += r[lt + st];
+		fx_group_sync(G, gid);
+	}
+	return r[0];
+}
+
+/* Reduced density matrix over the k low qubits, ro[a][a'] = inv * sum over b of
+ * x[b, a] conj(x[b, a']), by `nt` threads: 2x2 blocks of the lower triangle (4
+ * amplitudes read for 4 products) written with their mirror image, each by S
+ * lanes that share the b of small matrices. */
+template <typename F>
+__device__ __forceinline__ void fx_rho(F amp, uint32_t n, uint32_t k, double inv, double total,
+				       double2 *ro, uint32_t thread, uint32_t nt)
+{
+	const uint32_t dim = 1u << k, K = 1u << (n - k);
+	if (k == 0) {
+		if (thread == 0)
+			ro[0] = make_double2(total * inv, 0.0);
+		return;
+	}
+	const uint32_t nb = dim >> 1, nblk = nb * (nb + 1) / 2;
+	uint32_t S = 1;
+	while (S < 32u && S < nt && S < K && nblk * S < nt)
+		S <<= 1;
+	const uint32_t share = thread & (S - 1u);
+	const uint32_t lanes =
+		S == 32u ? 0xffffffffu : ((1u << S) - 1u) << (threadIdx.x & 31u & ~(S - 1u));
+	for (uint32_t x = thread / S; x < nblk; x += nt / S) {
+		uint32_t i = (uint32_t)((sqrtf(8.0f * (float)x + 1.0f) - 1.0f) * 0.5f);
+		while ((i + 1) * (i + 2) / 2 <= x)
+			++i;
+		while (i * (i + 1) / 2 > x)
+			--i;
+		const uint32_t a = 2 * i, c = 2 * (x - i * (i + 1) / 2);
+		double re[2][2] = { { 0.0, 0.0 }, { 0.0, 0.0 } }, im[2][2] = { { 0.0, 0.0 }, { 0.0, 0.0 } };
+#pragma unroll 4
+		for (uint32_t b = share; b < K; b += S) {
+			const double2 u[2] = { amp((b << k) | a), amp((b << k) | a | 1u) };
+			const double2 v[2] = { amp((b << k) | c), amp((b << k) | c | 1u) };
+#pragma unroll
+			for (int p = 0; p < 2; ++p)
+#pragma unroll
+				for (int q = 0; q < 2; ++q) {
+					re[p][q] = fma(u[p].x, v[q].x, fma(u[p].y, v[q].y, re[p][q]));
+					im[p][q] = fma(u[p].y, v[q].x, fma(-u[p].x, v[q].y, im[p][q]));
+				}
+		}
+#pragma unroll
+		for (int p = 0; p < 2; ++p)
+#pragma unroll
+			for (int q = 0; q < 2; ++q) {
+				for (uint32_t d = S >> 1; d > 0; d >>= 1) {
+					re[p][q] += __shfl_xor_sync(lanes, re[p][q], d);
+					im[p][q] += __shfl_xor_sync(lanes, im[p][q], d);
+				}
+				const uint32_t r = a + p, s = c + q;
+				if (share || r < s)
+					continue; /* a diagonal block's own mirror image */
+				const double x0 = re[p][q] * inv, y0 = r == s ? 0.0 : im[p][q] * inv;
+				ro[(size_t)r * dim + s] = make_double2(x0, y0);
+				if (r != s)
+					ro[(size_t)s * dim + r] = make_double2(x0, -y0);
+			}
+	}
+}
+
+/* Registers of n <= 12 qubits: each in the shared memory of G = 2^(n - 4)
+ * threads, one register to a warp below 32 (several to a warp ran their circuits
+ * one after the other: 2 ms for 64 registers of 4 qubits, now 0.3 for all below
+ * 9).  Latency bound: a chain of passes, each with a few operations.  The
+ * programs are read once, operation by operation, so the group first touches all
+ * of a program (it then lies in the L1 cache). */
+template <typename R, int SW, int MINB>
+__global__ void __launch_bounds__(kFxThreads, MINB)
+	k_batch_fx(const unsigned char *__restrict__ blob, const dk_breg *__restrict__ regs, int nregs,
+		   int n, typename CT<R>::T *states, double2 *rho_out, int keep_states)
+{
+	typedef typename CT<R>::T C2;
+	extern __shared__ __align__(16) unsigned char sm[];
+	__shared__ double red[kFxThreads];
+	const int G = 1 << (n - DK_FX_BITS), width = G < 32 ? 32 : G;
+	const int gid = threadIdx.x / width;
+	const uint32_t lt = threadIdx.x % width, lane = lt & 31u, warp = lt >> 5;
+	const uint32_t T = 1u << n;
+	unsigned char *const tile = sm + (size_t)gid * T * sizeof(C2);
+	C2 *const amps = reinterpret_cast<C2 *>(tile);
+
+	const int r = blockIdx.x * (kFxThreads / width) + gid;
+	if (r < nregs && (int)lt < G) {
+		const dk_breg reg = regs[r];
+		const unsigned char *prog = blob + reg.prog;
+		/* |0..0>: the layout maps index 0 to slot 0 */
+		for (uint32_t i = lt; i < T; i += G)
+			amps[i] = mk((R)(i == 0 ? 1 : 0), (R)0);
+		fx_group_sync(G, gid);
+		for (uint32_t s = 0; s < reg.nsweep; ++s) {
+			const dk_sweep_hdr *h = reinterpret_cast<const dk_sweep_hdr *>(prog);
+			const uint32_t bytes = __ldg(&h->bytes);
+			for (uint32_t i = 128u * lt; i < bytes; i += 128u * (uint32_t)G) {
+				uint32_t x;
+				asm volatile("ld.global.nc.b32 %0, [%1];" : "=r"(x) : "l"(prog + i));
+			}
+			const int npass = __ldg(&h->npass);
+			const dk_fx_pass *passes =
+				reinterpret_cast<const dk_fx_pass *>(prog + sizeof(dk_sweep_hdr));
+			const uint4 *lists = reinterpret_cast<const uint4 *>(passes + npass);
+			const uint4 *ops = reinterpret_cast<const uint4 *>(prog + __ldg(&h->gate_off));
+			const uint4 *table = reinterpret_cast<const uint4 *>(prog + __ldg(&h->mat_off));
+			for (int p = 0; p < npass; ++p) {
+				const dk_fx_pass *pd = passes + p;
+				/* no tile conditions: one list */
+				const uint4 ph = __ldg(reinterpret_cast<const uint4 *>(pd));
+				const uint4 l0 = __ldg(lists + 2 * ph.y), l1 = __ldg(lists + 2 * ph.y + 1);
+				if (l1.w && !(ph.x & DK_FX_STORE))
+					continue;
+				const uint32_t sg = __ldg(&pd->slo[lane]) ^ __ldg(&pd->shi[warp]);
+				C2 a[DK_FX_REGS];
+				auto slot = [&](int q, uint32_t base, uint32_t x, uint32_t y) -> uint32_t {
+					return base ^ ((q & 1) ? x & 0xffffu : 0u) ^ ((q & 2) ? x >> 16 : 0u) ^
+					       ((q & 4) ? y & 0xffffu : 0u) ^ ((q & 8) ? y >> 16 : 0u);
+				};
+				const uint32_t gb = sg ^ (l1.x & 0xffffu), sb = sg ^ (l1.x >> 16);
+#pragma unroll
+				for (int q = 0; q < DK_FX_REGS; ++q)
+					a[q] = *reinterpret_cast<const C2 *>(tile + slot(q, gb, l0.x, l0.y));
+				const uint32_t raw = (ph.x & DK_PASS_CTL)
+							     ? (__ldg(&pd->rlo[lane]) | __ldg(&pd->rhi[warp]))
+							     : 0u;
+				const uint32_t o1 = l1.y >> 16;
+				for (uint32_t o = l1.y & 0xffffu; o < o1; ++o) {
+					const uint4 d = __ldg(ops + o);
+					if ((d.z | d.w) && !ctl_ok(raw, d.z, d.w))
+						continue;
+					fx_op<true>(a, d.x & 0xffffu, d.x >> 16, table + d.y);
+				}
+#pragma unroll
+				for (int q = 0; q < DK_FX_REGS; ++q)
+					*reinterpret_cast<C2 *>(tile + slot(q, sb, l0.z, l0.w)) = a[q];
+				if ((ph.x & DK_PASS_WARP) && G >= 64)
+					__syncwarp();
+				else
+					fx_group_sync(G, gid);
+			}
+			prog += bytes;
+		}
+		auto amp = [&](uint32_t i) -> double2 { return to_c128(amps[swz<SW>(i)]); };
+		double part = 0.0;
+		for (uint32_t i = lt; i < T; i += G) {
+			if (keep_states)
+				states[reg.state + i] = amps[swz<SW>(i)];
+			part += sqabs(amp(i));
+		}
+		const double total = fx_group_sum(part, G, gid, lt, red + gid * width);
+		fx_rho(amp, (uint32_t)n, reg.keep, 1.0 / total, total, rho_out + reg.rho, lt, (uint32_t)G);
+	}
+}
+
+__device__ __forceinline__ void cluster_sync()
+{
+	/* device-scope fences: the CTAs exchange the register through global memory */
+	__threadfence();
+	asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::
+			     : "memory");
+	__threadfence();
+}
+
+/* Registers of 13-16 qubits: a cluster each, one CTA per tile up to 8.  Bound by
+ * the latency of the passes' operations (47 % of the issue slots used, 2.5 of 3
+ * CTAs per SM resident), so a circuit's length counts as much as the work: one CTA
+ * for all tiles of a register made a batch as long as its longest circuit.  1024
+ * circuits of 4-16 qubits, complex64: 4.25 ms (18 with one CTA per register gate by
+ * gate); the 86 registers of 16 qubits among them 2.7 ms, of which the matrices
+ * take 0.7; with clusters of 4 CTAs 3.3, of 2 5.4. */
+template <typename R, int MINB, bool NARROW>
+__global__ void __launch_bounds__(kFxThreads, MINB)
+	k_batch_cluster(const unsigned char *__restrict__ blob, const dk_breg *__restrict__ regs,
+			typename CT<R>::T *states, double2 *rho_out)
+{
+	typedef typename CT<R>::T C2;
+	extern __shared__ __align__(16) unsigned char sm[];
+	__shared__ double red[kFxThreads];
+	uint32_t rank, size;
+	asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+	asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(size));
+	const uint32_t tid = rank * blockDim.x + threadIdx.x, nt = size * blockDim.x;
+	const dk_breg reg = regs[blockIdx.x / size];
+	C2 *gs = states + reg.state;
+	const uint32_t T = 1u << reg.n;
+	const unsigned char *prog = blob + reg.prog;
+	for (uint32_t i = tid; i < T; i += nt)
+		gs[i] = mk((R)(i == 0 ? 1 : 0), (R)0);
+	cluster_sync();
+	for (uint32_t s = 0; s < reg.nsweep; ++s) {
+		const uint32_t bytes = __ldg(&reinterpret_cast<const dk_sweep_hdr *>(prog)->bytes);
+		double x = 0.0, y = 0.0;
+		fx_sweep<R, NARROW>(gs, gs, prog, sm, rank, size, 0, x, y);
+		cluster_sync();
+		prog += bytes;
+	}
+	auto amp = [&](uint32_t i) -> double2 { return to_c128(gs[i]); };
+	double part = 0.0;
+	for (uint32_t i = threadIdx.x; i < T; i += blockDim.x)
+		part += sqabs(amp(i));
+	const double total = fx_group_sum(part, (int)blockDim.x, 0, threadIdx.x, red);
+	fx_rho(amp, reg.n, reg.keep, 1.0 / total, total, rho_out + reg.rho, tid, nt);
+}
+
 /* Per-register comparison of two batches of the same circuits (precision
  * form of the batch): fidelity |<x|y>|^2 / (<x|x> <y|y>) and the largest
  * |x_i / |x| - y_i / |y||, in FP64, one CTA per register (states in each
@@ -293,7 +525,10 @@ __global__ void __launch_bounds__(256)
 namespace {
 
 struct BatchClass {
-	int m = 0;
+	int m = 0; /* tile bits */
+	int fx = 0; /* factored sweeps: 1 one tile, 2 a cluster per register */
+	uint32_t most = 0; /* bytes of the longest sweep program (fx = 2) */
+	unsigned qubits = 0; /* of its registers (fx = 2) */
 	std::vector<dk_breg> regs;
 	dk_breg *dregs = nullptr;
 };
@@ -383,6 +618,61 @@ static void batch_release_device(dk_batch *b)
 	b->drho = nullptr;
 }
 
+/* CTAs of a cluster: one per tile, 8 at most (the portable limit). */
+static int cluster_size(const BatchClass &cl)
+{
+	const int tiles = 1 << (cl.qubits - (unsigned)cl.m);
+	return tiles < 8 ? tiles : 8;
+}
+
+template <typename R, int MINB, bool NARROW>
+static cudaError_t enqueue_cluster(dk_batch *b, const BatchClass &cl, cudaStream_t st)
+{
+	typedef typename dk::CT<R>::T C2;
+	const int size = cluster_size(cl);
+	cudaLaunchConfig_t cfg = {};
+	cudaLaunchAttribute at[1];
+	at[0].id = cudaLaunchAttributeClusterDimension;
+	at[0].val.clusterDim.x = (unsigned)size;
+	at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+	cfg.gridDim = dim3((unsigned)(cl.regs.size() * size));
+	cfg.blockDim = dim3(NARROW ? 32u : 1u << (cl.m - DK_FX_BITS));
+	cfg.dynamicSmemBytes = (sizeof(C2) << cl.m) + cl.most;
+	cfg.stream = st;
+	cfg.attrs = at;
+	cfg.numAttrs = 1;
+	auto kern = dk::k_batch_cluster<R, MINB, NARROW>;
+	/* the most that any batch needs, so that no batch lowers another's */
+	cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+					     (int)((sizeof(C2) << 12) + DK_FX_BYTES_SMALL));
+	if (e != cudaSuccess)
+		return e;
+	return cudaLaunchKernelEx(&cfg, kern, (const unsigned char *)b->dblob,
+				  (const dk_breg *)cl.dregs, (C2 *)b->dstates, b->drho);
+}
+
+template <typename R, int SW, int MINB>
+static cudaError_t enqueue_factored(dk_batch *b, const BatchClass &cl, int keep_states,
+				    cudaStream_t st)
+{
+	typedef typename dk::CT<R>::T C2;
+	if (cl.fx == 2)
+		return cl.m < DK_FX_BITS + 5 ? enqueue_cluster<R, MINB, true>(b, cl, st)
+					     : enqueue_cluster<R, MINB, false>(b, cl, st);
+	const int nregs = (int)cl.regs.size();
+	const int per_cta = dk::kFxThreads >> (cl.m < DK_FX_BITS + 5 ? 5 : cl.m - DK_FX_BITS);
+	const size_t smem = (sizeof(C2) << cl.m) * per_cta;
+	auto kern = dk::k_batch_fx<R, SW, MINB>;
+	cudaError_t e =
+		cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+				     (int)(sizeof(C2) << 12));
+	if (e != cudaSuccess)
+		return e;
+	kern<<<(nregs + per_cta - 1) / per_cta, dk::kFxThreads, smem, st>>>(
+		b->dblob, cl.dregs, nregs, cl.m, (C2 *)b->dstates, b->drho, keep_states);
+	return cudaGetLastError();
+}
+
 extern "C" {
 
 static int batch_build(int precision, unsigned num_circuits, const unsigned *num_qubits,
@@ -420,7 +710,7 @@ static int batch_build(int precision, unsigned num_circuits, const unsigned *num
 	const size_t amp = precision == DK_C128 ? 16 : 8;
 	std::unique_ptr<unsigned char[]> blob; /* programs, uninitialised between them */
 	size_t blob_len = 0;
-	std::vector<int> class_of_m(13, -1);
+	std::vector<int> class_of(64, -1); /* by kind of planning and size */
 	b->rho_off.resize(num_circuits);
 	b->state_off.resize(num_circuits);
 	b->n.assign(num_qubits, num_qubits + num_circuits);
@@ -431,10 +721,47 @@ static int batch_build(int precision, unsigned num_circuits, const unsigned *num
 	 * programs are kept back to back in its own byte vector. */
 	struct Planned {
 		std::vector<unsigned char> prog;
-		uint32_t nsweep = 0;
+		uint32_t nsweep = 0, most = 0;
+		int fx = 0;
 		int rc = 0;
 	};
 	std::vector<Planned> planned(num_circuits);
+	/* 0: planned (or failed with *rc), 1: some gate has no factoring */
+	auto plan_factored = [](const std::vector<dk_flat_op> &flat, unsigned n, int prec, int m,
+				std::vector<unsigned char> *prog, uint32_t *nsweep, uint32_t *most,
+				int *fx, int *rc) -> int {
+		dk_plan_limits lim = {};
+		lim.tile_bits = m;
+		dk_plan_default_limits(prec, n, &lim);
+		lim.tile_bits = m;
+		dk_fx_plan *fp = nullptr;
+		*rc = dk_fx_begin(flat.data(), (int)flat.size(), n, prec, &lim, &fp);
+		if (*rc)
+			return 0;
+		if (!dk_fx_all(fp)) {
+			dk_fx_end(fp);
+			return 1;
+		}
+		dk_step step;
+		const unsigned char *src;
+		int more;
+		while ((more = dk_fx_next(fp, &step, &src)) > 0) {
+			const uint32_t bytes = ((const dk_sweep_hdr *)src)->bytes;
+			try {
+				prog->insert(prog->end(), src, src + bytes);
+			} catch (...) {
+				more = -DK_ERR_ALLOC;
+				break;
+			}
+			++*nsweep;
+			if (bytes > *most)
+				*most = bytes;
+		}
+		dk_fx_end(fp);
+		*fx = 1;
+		*rc = more < 0 ? -more : 0;
+		return 0;
+	};
 	auto plan_some = [&](unsigned first, unsigned stride) {
 		std::vector<dk_gate> gates;
 		std::vector<dk_flat_op> flat;
@@ -473,6 +800,10 @@ static int batch_build(int precision, unsigned num_circuits, const unsigned *num
 			lim.tile_bits = m;
 			if (lim.low_bits > m - 3)
 				lim.low_bits = m - 3;
+			/* factored sweeps when every gate has a factoring */
+			if (!plan_factored(flat, n, precision, m, &pl.prog, &pl.nsweep, &pl.most, &pl.fx,
+					   &pl.rc))
+				continue;
 			dk_plan plan;
 			pl.rc = dk_plan_build(flat.data(), (int)flat.size(), n, precision, &lim, &plan);
 			if (pl.rc)
@@ -566,17 +897,33 @@ static int batch_build(int precision, unsigned num_circuits, const unsigned *num
 		b->rho_off[c] = b->rho_elems;
 		b->state_amps += 1ull << n;
 		b->rho_elems += 1ull << (2 * keep);
-		if (class_of_m[m] < 0) {
-			class_of_m[m] = (int)b->classes.size();
+		/* 0-12: gate by gate, by tile; 16-28: one factored tile; 32-48: a
+		 * cluster, by size */
+		const int fx = !planned[c].fx ? 0 : n <= 12 ? 1 : 2;
+		const int key = fx == 0 ? m : 16 * fx + (int)n;
+		if (class_of[key] < 0) {
+			class_of[key] = (int)b->classes.size();
 			b->classes.emplace_back();
 			b->classes.back().m = m;
+			b->classes.back().fx = fx;
+			b->classes.back().qubits = n;
 		}
-		b->classes[class_of_m[m]].regs.push_back(reg);
+		BatchClass &cl = b->classes[class_of[key]];
+		cl.regs.push_back(reg);
+		if (planned[c].most > cl.most)
+			cl.most = planned[c].most;
 	}
-	/* larger registers first inside a class (better tail balance) */
+	/* larger registers and longer circuits first, in a class and among the
+	 * classes (better tail balance) */
 	for (auto &cl : b->classes)
 		std::stable_sort(cl.regs.begin(), cl.regs.end(),
-				 [](const dk_breg &x, const dk_breg &y) { return x.n > y.n; });
+				 [](const dk_breg &x, const dk_breg &y) {
+					 return x.n != y.n ? x.n > y.n : x.nsweep > y.nsweep;
+				 });
+	std::stable_sort(b->classes.begin(), b->classes.end(),
+			 [](const BatchClass &x, const BatchClass &y) {
+				 return x.regs[0].n > y.regs[0].n;
+			 });
 	const auto t2 = clk::now();
 	cudaError_t e = cudaMalloc(&b->dblob, blob_len ? blob_len : 16);
 	if (e == cudaSuccess && blob_len)
@@ -676,22 +1023,28 @@ static cudaError_t batch_enqueue(dk_batch *b, int keep_states)
 		e = cudaStreamWaitEvent(s2, fork, 0);
 		if (e != cudaSuccess)
 			break;
-		const int G = 1 << (cl.m - DK_PASS_BITS);
-		const int groups_per_cta = dk::kBatchThreads / G;
-		const size_t smem = batch_smem(b->prec, cl.m);
-		const int nregs = (int)cl.regs.size();
-		int blocks = (nregs + groups_per_cta - 1) / groups_per_cta;
-		const int cap = b->num_sms * b->ctas_per_sm;
-		if (blocks > cap)
-			blocks = cap;
-		if (b->prec == DK_C128)
-			dk::k_batch<double, 3><<<blocks, dk::kBatchThreads, smem, s2>>>(
-				b->dblob, cl.dregs, nregs, cl.m, (double2 *)b->dstates, b->drho,
-				keep_states);
-		else
-			dk::k_batch<float, 4><<<blocks, dk::kBatchThreads, smem, s2>>>(
-				b->dblob, cl.dregs, nregs, cl.m, (float2 *)b->dstates, b->drho,
-				keep_states);
+		if (cl.fx) {
+			e = b->prec == DK_C128
+				    ? enqueue_factored<double, 3, 2>(b, cl, keep_states, s2)
+				    : enqueue_factored<float, 4, 3>(b, cl, keep_states, s2);
+		} else {
+			const int G = 1 << (cl.m - DK_PASS_BITS);
+			const int groups_per_cta = dk::kBatchThreads / G;
+			const size_t smem = batch_smem(b->prec, cl.m);
+			const int nregs = (int)cl.regs.size();
+			int blocks = (nregs + groups_per_cta - 1) / groups_per_cta;
+			const int cap = b->num_sms * b->ctas_per_sm;
+			if (blocks > cap)
+				blocks = cap;
+			if (b->prec == DK_C128)
+				dk::k_batch<double, 3><<<blocks, dk::kBatchThreads, smem, s2>>>(
+					b->dblob, cl.dregs, nregs, cl.m, (double2 *)b->dstates, b->drho,
+					keep_states);
+			else
+				dk::k_batch<float, 4><<<blocks, dk::kBatchThreads, smem, s2>>>(
+					b->dblob, cl.dregs, nregs, cl.m, (float2 *)b->dstates, b->drho,
+					keep_states);
+		}
 		if (e == cudaSuccess)
 			e = cudaGetLastError();
 		if (e == cudaSuccess)

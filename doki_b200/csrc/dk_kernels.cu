@@ -1249,6 +1249,23 @@ __global__ void __launch_bounds__(256, 2)
 
 #include "dk_sweep_fx.cuh"
 
+template <typename R, int MINB, bool NARROW>
+__global__ void __launch_bounds__(256, MINB)
+	k_sweep_fx(const typename CT<R>::T *__restrict__ in, typename CT<R>::T *out,
+		   const unsigned char *__restrict__ prog, int sums, double *partials)
+{
+	extern __shared__ __align__(16) unsigned char sm[];
+	double insq = 0.0, outsq = 0.0;
+	fx_sweep<R, NARROW>(in, out, prog, sm, blockIdx.x, gridDim.x, sums, insq, outsq);
+	if (!sums)
+		return;
+	block_sum2(insq, outsq);
+	if (threadIdx.x == 0) {
+		partials[2 * blockIdx.x] = insq;
+		partials[2 * blockIdx.x + 1] = outsq;
+	}
+}
+
 enum { FIN_GATE = 0, FIN_COLLAPSE = 1, FIN_RESET = 2 };
 
 /* Sum the (in, out) partials of `nb` blocks in a fixed order and update the

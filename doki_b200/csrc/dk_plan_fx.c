@@ -205,6 +205,7 @@ struct dk_fx_plan {
 	int prec;
 	int nops; /* gates to plan */
 	int ngone; /* gates absorbed by others, not yet counted in a step */
+	int all; /* every gate has a factoring */
 	dk_plan_limits lim;
 	int *rem, head; /* gates left: rem[head .. nops) */
 	int *take, *order, *win; /* a sweep's gates; in pass order; a pass's leftovers */
@@ -1343,6 +1344,7 @@ int dk_fx_begin(const dk_flat_op *ops, int nops, unsigned n, int prec,
 		all &= P->g[i].kind != FX_NONE;
 	}
 	/* gates that dk_plan.c plans from their matrices take no factor */
+	P->all = all;
 	if (all)
 		move_factors(P);
 	P->nops = 0;
@@ -1361,6 +1363,8 @@ int dk_fx_begin(const dk_flat_op *ops, int nops, unsigned n, int prec,
 	*out = P;
 	return DK_OK;
 }
+
+int dk_fx_all(const dk_fx_plan *P) { return P->all; }
 
 void dk_fx_end(dk_fx_plan *P)
 {

@@ -1,6 +1,6 @@
 /*
- * The factored sweep kernel (included by dk_kernels.cu; programs from
- * dk_plan_fx.c, layout in dk_internal.h).
+ * The factored sweep (kernel in dk_kernels.cu, batches in dk_batch.cu; programs
+ * from dk_plan_fx.c, layout in dk_internal.h).
  *
  * A tile of 2^m amplitudes (12 bits: 64 or 32 KiB) comes into shared memory by
  * cp.async and goes through the passes of the program; thread t holds 16
@@ -23,6 +23,10 @@
  */
 #ifndef DK_SWEEP_FX_CUH_
 #define DK_SWEEP_FX_CUH_
+
+#ifndef DK_IN_BOUNDS /* translation units without index checks */
+#define DK_IN_BOUNDS(i, lim, site) true
+#endif
 
 /* Rotation of the 8 register pairs (p, p ^ V): a[p] += x a[q], a[q] += y a[p]
  * with the pair's real coefficients.  complex64 takes each pair's two
@@ -100,10 +104,9 @@ __device__ __forceinline__ void fx_swap(C2 (&a)[DK_FX_REGS], uint32_t mask)
 	}
 }
 
-/* 16 bytes of coefficients from shared memory.  Volatile, so that a batch of
- * them is requested before the arithmetic that the caller writes behind it:
- * loaded one by one at their use, each would cost the latency of a shared load
- * (a stage took 1100 cycles that way, 2 warps per scheduler). */
+/* 16 bytes of coefficients.  Volatile, so that a batch of them is requested
+ * before the arithmetic that the caller writes behind it.  `at` is an address in
+ * shared memory, or (GLOBAL) a pointer. */
 __device__ __forceinline__ void fx_load(double2 &v, uint32_t at)
 {
 	asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(at));
@@ -114,9 +117,33 @@ __device__ __forceinline__ void fx_load(float4 &v, uint32_t at)
 		     : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
 		     : "r"(at));
 }
+__device__ __forceinline__ void fx_load(double2 &v, const unsigned char *at)
+{
+	asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(at));
+}
+__device__ __forceinline__ void fx_load(float4 &v, const unsigned char *at)
+{
+	asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+		     : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+		     : "l"(at));
+}
+template <bool GLOBAL> struct FxAddr;
+template <> struct FxAddr<false> {
+	static __device__ __forceinline__ uint32_t of(const uint4 *p)
+	{
+		return (uint32_t)__cvta_generic_to_shared(p);
+	}
+};
+template <> struct FxAddr<true> {
+	static __device__ __forceinline__ const unsigned char *of(const uint4 *p)
+	{
+		return reinterpret_cast<const unsigned char *>(p);
+	}
+};
 
 /* a[4 b .. 4 b + 3] *= the diagonal's values, a batch of four ahead */
-__device__ __forceinline__ void fx_diag(double2 (&a)[DK_FX_REGS], uint32_t at)
+template <typename A>
+__device__ __forceinline__ void fx_diag(double2 (&a)[DK_FX_REGS], A at)
 {
 	double2 c[2][4];
 #pragma unroll
@@ -133,7 +160,8 @@ __device__ __forceinline__ void fx_diag(double2 (&a)[DK_FX_REGS], uint32_t at)
 			a[4 * b + i] = cmul(c[b & 1][i], a[4 * b + i]);
 	}
 }
-__device__ __forceinline__ void fx_diag(float2 (&a)[DK_FX_REGS], uint32_t at)
+template <typename A>
+__device__ __forceinline__ void fx_diag(float2 (&a)[DK_FX_REGS], A at)
 {
 	float4 c[2][2];
 #pragma unroll
@@ -154,14 +182,14 @@ __device__ __forceinline__ void fx_diag(float2 (&a)[DK_FX_REGS], uint32_t at)
 	}
 }
 
-template <typename C2>
+template <bool GLOBAL, typename C2>
 __device__ __forceinline__ void fx_op(C2 (&a)[DK_FX_REGS], uint32_t code, uint32_t mask,
 				      const uint4 *co)
 {
 	typedef typename FxCoef<C2>::T W;
 	const C2 *c = reinterpret_cast<const C2 *>(co);
 	if (code == DK_FX_STAGE) {
-		const uint32_t at = (uint32_t)__cvta_generic_to_shared(co);
+		const auto at = FxAddr<GLOBAL>::of(co);
 		W w[4];
 #pragma unroll
 		for (int i = 0; i < 4; ++i)
@@ -212,13 +240,17 @@ __device__ __forceinline__ void fx_op(C2 (&a)[DK_FX_REGS], uint32_t code, uint32
 	}
 }
 
-template <typename R, int MINB, bool NARROW>
-__global__ void __launch_bounds__(256, MINB)
-	k_sweep_fx(const typename CT<R>::T *__restrict__ in, typename CT<R>::T *out,
-		   const unsigned char *__restrict__ prog, int sums, double *partials)
+/* One sweep: the tiles first, first + step, ... of the register.  `sm` holds a
+ * tile and the program.  Sums of |amp|^2 of the tiles read (where tiles are
+ * skipped) and written go to insq and outsq. */
+template <typename R, bool NARROW>
+__device__ __forceinline__ void fx_sweep(const typename CT<R>::T *__restrict__ in,
+					 typename CT<R>::T *out,
+					 const unsigned char *__restrict__ prog, unsigned char *sm,
+					 uint64_t first, uint64_t step, int sums, double &insq,
+					 double &outsq)
 {
 	typedef typename CT<R>::T C2;
-	extern __shared__ __align__(16) unsigned char sm[];
 	__shared__ uint64_t sdep[DK_DEP_NIBBLES][16];
 	/* byte offsets in the register: of stream bit j, of the last pass's bit j */
 	__shared__ uint64_t soff[DK_FX_BITS], poff[DK_FX_BITS];
@@ -302,12 +334,12 @@ __global__ void __launch_bounds__(256, MINB)
 		}
 		return __ballot_sync(0xffffffffu, on);
 	};
-	/* the first tile >= t, stepping by the grid, that some gate acts on; its
+	/* the first tile t, t + step, ... that some gate acts on; its
 	 * base and conditions */
 	uint64_t base = 0;
 	uint32_t cmask = 0;
 	auto find_tile = [&](uint64_t t) -> uint64_t {
-		for (; t < ntiles; t += gridDim.x) {
+		for (; t < ntiles; t += step) {
 			base = tile_base(t);
 			cmask = cond_mask(base);
 			if (!skip_idle || cmask)
@@ -353,8 +385,7 @@ __global__ void __launch_bounds__(256, MINB)
 		}
 	};
 
-	double insq = 0.0, outsq = 0.0;
-	uint64_t t = find_tile(blockIdx.x);
+	uint64_t t = find_tile(first);
 	if (t < ntiles)
 		prefetch();
 	while (t < ntiles) {
@@ -395,7 +426,7 @@ __global__ void __launch_bounds__(256, MINB)
 					/* the results of this pass go to the register: once every
 					 * thread has gathered, the next tile's copy can start */
 					__syncthreads();
-					t = find_tile(t + gridDim.x);
+					t = find_tile(t + step);
 					if (t < ntiles)
 						prefetch();
 				}
@@ -406,7 +437,7 @@ __global__ void __launch_bounds__(256, MINB)
 					const uint4 d = *o;
 					if ((d.z | d.w) && !ctl_ok(raw, d.z, d.w))
 						continue;
-					fx_op(a, d.x & 0xffffu, d.x >> 16, table + d.y);
+					fx_op<false>(a, d.x & 0xffffu, d.x >> 16, table + d.y);
 				}
 				if (out_now) {
 					const uint64_t p0 = poff[0], p1 = poff[1], p2 = poff[2],
@@ -443,7 +474,7 @@ __global__ void __launch_bounds__(256, MINB)
 		if (!store) {
 			read16(stid, sro[0], sro[1], sro[2], sro[3]);
 			__syncthreads(); /* the buffer is free: start the next tile's copy */
-			t = find_tile(t + gridDim.x);
+			t = find_tile(t + step);
 			if (t < ntiles)
 				prefetch();
 			g0 = soff[0];
@@ -465,13 +496,6 @@ __global__ void __launch_bounds__(256, MINB)
 		}
 	}
 	cp_async_wait_all();
-	if (!sums)
-		return;
-	block_sum2(insq, outsq);
-	if (tid == 0) {
-		partials[2 * blockIdx.x] = insq;
-		partials[2 * blockIdx.x + 1] = outsq;
-	}
 }
 
 #endif

@@ -244,8 +244,12 @@ int dk_batch_build(int precision, unsigned num_circuits, const unsigned *num_qub
  * them one by one, each gate charged its arithmetic plus `fold` FP64
  * multiply-adds per thread of dispatch; 0 = the planner's default (96),
  * < 0 = off (every gate applied on its own), larger values fold more
- * readily.  The circuits are planned on all host cores.
- * CTAs per SM for the batch kernels (1..4); the autotuner's second knob. */
+ * readily.  Circuits whose gates all have a factoring (diagonal, anti-diagonal
+ * or one-qubit matrices, any controls) run as factored sweeps, which take
+ * neither `fold` nor the CTAs per SM below.  The circuits are planned on all
+ * host cores.
+ * CTAs per SM for the gate-by-gate batch kernel (1..4); the autotuner's second
+ * knob. */
 int dk_batch_set_ctas(dk_batch *b, int ctas_per_sm);
 /* Queue every circuit (captured into a CUDA graph on first use); keep_states
  * also stores each final register for dk_batch_state.  Returns before the
