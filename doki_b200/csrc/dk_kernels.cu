@@ -1951,15 +1951,72 @@ __device__ __forceinline__ uint64_t deposit(uint64_t v, uint64_t mask)
 	return r;
 }
 
+/* M[b << k | a] = the amplitude at (a on the kept qubits, b on the traced ones),
+ * widened to FP64: a permutation of index bits.  A CTA moves tiles of the index
+ * bits that are among the 5 lowest of the register or of M, through shared
+ * memory, so that both sides see runs of 32 amplitudes.  Memory bound: 25 qubits,
+ * 9 scattered ones kept, complex64: 186 us for 805 MB (805 us with an index of
+ * its own and an uncoalesced read per element of M). */
+constexpr int kGatherBits = 10;
+
+struct GatherMap {
+	uint64_t in[kGatherBits], out[kGatherBits]; /* offset of tile bit j, in order of either side */
+	uint16_t slot_in[kGatherBits]; /* shared-memory slot of the input side's bit j */
+	uint8_t from[64], to[64]; /* the other index bits: of the register, of M */
+	int bits, rest;
+};
+
+__host__ __device__ __forceinline__ uint32_t gather_slot(uint32_t x)
+{
+	return x ^ (x >> 5); /* lanes along the upper bits, too, take distinct banks */
+}
+
 template <typename R>
 __global__ void __launch_bounds__(256)
-	k_gather_kept(const typename CT<R>::T *__restrict__ d, uint64_t keep,
-		      uint64_t trace, int k, uint64_t total, double2 *M)
+	k_gather_kept(const typename CT<R>::T *__restrict__ d, const GatherMap map, uint64_t ntiles,
+		      double2 *M)
 {
-	for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-	     e += (uint64_t)gridDim.x * blockDim.x) {
-		const uint64_t a = e & ((1ull << k) - 1ull), b = e >> k;
-		M[e] = to_c128(d[deposit(a, keep) | deposit(b, trace)]);
+	typedef typename CT<R>::T C2;
+	__shared__ C2 tile[1 << kGatherBits];
+	constexpr int kPer = (1 << kGatherBits) / 256;
+	const uint32_t lane = threadIdx.x & 31u, T = 1u << map.bits;
+	uint64_t in[kPer], out[kPer];
+	uint32_t si[kPer];
+#pragma unroll
+	for (int r = 0; r < kPer; ++r) {
+		const uint32_t e = threadIdx.x + 256u * r;
+		in[r] = out[r] = 0;
+		si[r] = 0;
+#pragma unroll
+		for (int j = 0; j < kGatherBits; ++j)
+			if ((e >> j) & 1u) {
+				in[r] |= map.in[j];
+				out[r] |= map.out[j];
+				si[r] ^= map.slot_in[j];
+			}
+	}
+	const bool lo = (int)lane < map.rest, hi = (int)lane + 32 < map.rest;
+	const uint64_t f0 = lo ? 1ull << map.from[lane] : 0, t0 = lo ? 1ull << map.to[lane] : 0;
+	const uint64_t f1 = hi ? 1ull << map.from[lane + 32] : 0, t1 = hi ? 1ull << map.to[lane + 32] : 0;
+	auto spread = [&](uint64_t x, uint64_t v0, uint64_t v1) -> uint64_t {
+		const uint64_t v = (((x >> lane) & 1ull) ? v0 : 0) | (((x >> (lane + 32)) & 1ull) ? v1 : 0);
+		return ((uint64_t)__reduce_or_sync(0xffffffffu, (uint32_t)(v >> 32)) << 32) |
+		       __reduce_or_sync(0xffffffffu, (uint32_t)v);
+	};
+	for (uint64_t x = blockIdx.x; x < ntiles; x += gridDim.x) {
+		const uint64_t src = spread(x, f0, f1), dst = spread(x, t0, t1);
+#pragma unroll
+		for (int r = 0; r < kPer; ++r)
+			if (threadIdx.x + 256u * r < T)
+				tile[si[r]] = __ldcs(d + (src | in[r]));
+		__syncthreads();
+#pragma unroll
+		for (int r = 0; r < kPer; ++r) {
+			const uint32_t e = threadIdx.x + 256u * r;
+			if (e < T)
+				M[dst | out[r]] = to_c128(tile[gather_slot(e)]);
+		}
+		__syncthreads();
 	}
 }
 
@@ -2160,8 +2217,10 @@ __global__ void __launch_bounds__(256)
 	}
 }
 
-/* C = alpha * sum over s (in order) of part[s], on the lower tiles */
-__global__ void __launch_bounds__(256)
+/* C = alpha * sum over s (in a fixed order) of part[s], on the lower tiles: one
+ * element per thread, eight partials requested at a time (128 x 128, 64 partials:
+ * 10.6 us; 68 with four elements in turn per thread and one load in flight). */
+__global__ void __launch_bounds__(128)
 	k_rho_reduce(const double2 *__restrict__ part, int nsplit, uint64_t dim, double alpha,
 		     double2 *C)
 {
@@ -2172,7 +2231,19 @@ __global__ void __launch_bounds__(256)
 		if (a / kRhoTile < c / kRhoTile)
 			continue;
 		double x = 0.0, y = 0.0;
-		for (int s2 = 0; s2 < nsplit; ++s2) {
+		int s2 = 0;
+		for (; s2 + 8 <= nsplit; s2 += 8) {
+			double2 v[8];
+#pragma unroll
+			for (int j = 0; j < 8; ++j)
+				v[j] = __ldcs(part + (uint64_t)(s2 + j) * total + e);
+#pragma unroll
+			for (int j = 0; j < 8; ++j) {
+				x += v[j].x;
+				y += v[j].y;
+			}
+		}
+		for (; s2 < nsplit; ++s2) {
 			const double2 v = part[(uint64_t)s2 * total + e];
 			x += v.x;
 			y += v.y;
@@ -2996,15 +3067,45 @@ cudaError_t launch_gather_kept(int prec, const void *d, unsigned n,
 		g_launches += 1;
 		return cudaGetLastError();
 	}
-	const int blocks = grid_for(total, 256 * 4, g_num_sms * 8);
+	/* from[j]: the register's bit that is bit j of M */
+	uint8_t from[64], to[64];
+	int nb = 0;
+	for (int side = 0; side < 2; ++side)
+		for (unsigned q = 0; q < n; ++q)
+			if ((((side ? trace : keep_mask) >> q) & 1ull) != 0) {
+				from[nb] = (uint8_t)q;
+				to[q] = (uint8_t)nb++;
+			}
+	GatherMap map;
+	memset(&map, 0, sizeof(map));
+	uint64_t in_tile = 0; /* of the register's bits */
+	map.bits = n < (unsigned)kGatherBits ? (int)n : kGatherBits;
+	for (unsigned j = 0; j < 5 && j < n; ++j)
+		in_tile |= (1ull << j) | (1ull << from[j]);
+	for (unsigned q = 0; __builtin_popcountll(in_tile) < map.bits; ++q)
+		in_tile |= 1ull << q;
+	int ni = 0, no = 0;
+	uint8_t rank[64]; /* of a tile bit among M's */
+	for (unsigned j = 0; j < n; ++j)
+		if ((in_tile >> from[j]) & 1ull) {
+			rank[from[j]] = (uint8_t)no;
+			map.out[no++] = 1ull << j;
+		}
+	for (unsigned q = 0; q < n; ++q) {
+		if ((in_tile >> q) & 1ull) {
+			map.slot_in[ni] = (uint16_t)gather_slot(1u << rank[q]);
+			map.in[ni++] = 1ull << q;
+		} else {
+			map.from[map.rest] = (uint8_t)q;
+			map.to[map.rest++] = to[q];
+		}
+	}
+	const uint64_t ntiles = total >> map.bits;
+	const int blocks = grid_for(ntiles, 1, g_num_sms * 8);
 	if (prec == DK_C128)
-		k_gather_kept<double><<<blocks, 256, 0, st>>>((const double2 *)d,
-							     keep_mask, trace, k,
-							     total, M);
+		k_gather_kept<double><<<blocks, 256, 0, st>>>((const double2 *)d, map, ntiles, M);
 	else
-		k_gather_kept<float><<<blocks, 256, 0, st>>>((const float2 *)d,
-							    keep_mask, trace, k, total,
-							    M);
+		k_gather_kept<float><<<blocks, 256, 0, st>>>((const float2 *)d, map, ntiles, M);
 	g_launches += 1;
 	return cudaGetLastError();
 }
@@ -3043,13 +3144,14 @@ static cudaError_t rho_prepare(int *ctas_per_sm)
 	return err;
 }
 
-/* Traced-range splits of the reduced density product.  Tiles x splits CTAs
- * should fill whole waves of the resident CTA slots (a 1024 x 1024 result
- * has 136 tiles; 13 splits fill 12 waves of 148 at 99.5 %, where 8 would
- * leave the last of 8 waves a third full); each split keeps at least 256
- * traced values, there are at most 64 and their partials stay within 1 GiB.
- * Among split counts giving at least two waves, a larger count is taken only
- * when it fills the waves 2 % better. */
+/* Traced-range splits of the reduced density product: at most one per CTA slot,
+ * each with at least 256 traced values, their partials within 1 GiB.  Taken is the
+ * count with the shortest time, in slabs of kRhoSlab traced values (3.1 us of FP64
+ * MMAs): waves of CTAs times slabs of a CTA, 4 more for a CTA's start and its
+ * partial tile, and the partials' way through memory (20 MB per slab's time).  3
+ * tiles of 16384 traced values (128 x 128) take 49 splits, one wave, 49 us where
+ * 64 in two waves took 69; 36 tiles of 65536 (512 x 512) 4, 2.0 ms like 37, whose
+ * partials took another 0.1. */
 int rho_splits(uint64_t dim, uint64_t K, int num_sms)
 {
 	if (dim < (uint64_t)kRhoTile) {
@@ -3063,18 +3165,14 @@ int rho_splits(uint64_t dim, uint64_t K, int num_sms)
 	rho_prepare(&occ);
 	const uint64_t slots = (uint64_t)(num_sms > 0 ? num_sms : 1) * (uint64_t)occ;
 	const uint64_t part_cap = (1ull << 30) / (16 * dim * dim);
-	uint64_t best = 1;
-	double best_fill = -1.0;
-	for (uint64_t ns = 1; ns <= 64 && ns * 256 <= K && (ns == 1 || ns <= part_cap); ++ns) {
-		const uint64_t ctas = ntile * ns;
-		const bool more_allowed = ns < 64 && (ns + 1) * 256 <= K && ns + 1 <= part_cap;
-		if (ctas < 2 * slots && more_allowed)
-			continue;
-		const uint64_t waves = (ctas + slots - 1) / slots;
-		const double fill = (double)ctas / (double)(waves * slots);
-		if (fill > best_fill + 0.02) {
+	uint64_t best = 1, best_cost = ~0ull;
+	for (uint64_t ns = 1; ns <= slots && (ns == 1 || (ns * 256 <= K && ns <= part_cap)); ++ns) {
+		const uint64_t slabs = ((K + ns - 1) / ns + kRhoSlab - 1) / kRhoSlab;
+		const uint64_t cost = (ntile * ns + slots - 1) / slots * (slabs + 4) +
+				      ns * dim * dim * 32 / (20u << 20);
+		if (cost < best_cost) {
 			best = ns;
-			best_fill = fill;
+			best_cost = cost;
 		}
 	}
 	return (int)best;
@@ -3086,8 +3184,8 @@ cudaError_t launch_rho(const double2 *A, uint64_t dim, uint64_t K, double alpha,
 	if (dim < (uint64_t)kRhoTile) {
 		const uint64_t bchunk = (K + nsplit - 1) / nsplit;
 		k_rho_small<<<nsplit, 256, 0, st>>>(A, (uint32_t)dim, K, bchunk, part);
-		const int blocks = grid_for(dim * dim, 256, g_num_sms * 8);
-		k_rho_reduce<<<blocks, 256, 0, st>>>(part, nsplit, dim, alpha, C);
+		const int blocks = grid_for(dim * dim, 128, g_num_sms * 16);
+		k_rho_reduce<<<blocks, 128, 0, st>>>(part, nsplit, dim, alpha, C);
 		g_launches += 2;
 		return cudaGetLastError();
 	}
@@ -3101,8 +3199,8 @@ cudaError_t launch_rho(const double2 *A, uint64_t dim, uint64_t K, double alpha,
 	k_rho_tc<<<grid, 256, kRhoSmem, st>>>(A, dim, K, bchunk, nsplit == 1 ? C : part, alpha);
 	g_launches += 1;
 	if (nsplit > 1) {
-		const int blocks = grid_for(dim * dim, 256 * 4, g_num_sms * 8);
-		k_rho_reduce<<<blocks, 256, 0, st>>>(part, nsplit, dim, alpha, C);
+		const int blocks = grid_for(dim * dim, 128, g_num_sms * 16);
+		k_rho_reduce<<<blocks, 128, 0, st>>>(part, nsplit, dim, alpha, C);
 		g_launches += 1;
 	}
 	return cudaGetLastError();
