@@ -1250,20 +1250,44 @@ __global__ void __launch_bounds__(256, 2)
 
 #include "dk_sweep_fx.cuh"
 
+/* The last block to finish also makes the register's scalars out of all blocks'
+ * sums, in a fixed order (FIN_GATE of k_finalize, which as a launch of its own cost
+ * a flush 4 us on the device and 3 on the host).  `ticket` is 0 before and after. */
 template <typename R, int MINB, bool NARROW>
 __global__ void __launch_bounds__(256, MINB)
 	k_sweep_fx(const typename CT<R>::T *__restrict__ in, typename CT<R>::T *out,
-		   const unsigned char *__restrict__ prog, int sums, double *partials)
+		   const unsigned char *__restrict__ prog, int sums, int all, double *partials,
+		   unsigned *ticket, const dk_scal *sc_in, dk_scal *sc_out)
 {
 	extern __shared__ __align__(16) unsigned char sm[];
+	__shared__ bool last;
 	double insq = 0.0, outsq = 0.0;
 	fx_sweep<R, NARROW>(in, out, prog, sm, blockIdx.x, gridDim.x, sums, insq, outsq);
 	if (!sums)
 		return;
 	block_sum2(insq, outsq);
+	if (gridDim.x > 1) {
+		if (threadIdx.x == 0) {
+			__stcg(partials + 2 * blockIdx.x, insq);
+			__stcg(partials + 2 * blockIdx.x + 1, outsq);
+			__threadfence();
+			last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+			__threadfence();
+		}
+		__syncthreads();
+		if (!last)
+			return;
+		insq = outsq = 0.0;
+		for (unsigned i = threadIdx.x; i < gridDim.x; i += blockDim.x) {
+			insq += __ldcg(partials + 2 * i);
+			outsq += __ldcg(partials + 2 * i + 1);
+		}
+		block_sum2(insq, outsq);
+	}
 	if (threadIdx.x == 0) {
-		partials[2 * blockIdx.x] = insq;
-		partials[2 * blockIdx.x + 1] = outsq;
+		const double c = all ? outsq : sc_in->csq - insq + outsq;
+		sc_out->csq = c;
+		sc_out->norm = sqrt(c);
 	}
 }
 
@@ -1564,19 +1588,20 @@ __global__ void __launch_bounds__(256, 2)
 		for (uint32_t i = 0; i < (blockDim.x >> 5); ++i)
 			if ((i & wmask) == wmask)
 				t += red[i][col];
-	partials[(size_t)blockIdx.x * kPartialStride + q] = t;
+	partials[(size_t)q * gridDim.x + blockIdx.x] = t;
 }
 
 /* marg[q] = sum of the blocks' partials, in a fixed order: one block per
  * qubit (one thread per qubit took 136 us for the 2048 partials of a 24-qubit
- * register, longer than the pass over the register itself; this takes 5). */
+ * register, longer than the pass over the register itself; this takes 6.5, 7.2 with
+ * a block's partials side by side instead of a qubit's). */
 __global__ void __launch_bounds__(256)
 	k_marg_finalize(const double *partials, int nb, double *marg)
 {
 	const int q = blockIdx.x;
 	double t = 0.0, dummy = 0.0;
 	for (int b = threadIdx.x; b < nb; b += blockDim.x)
-		t += partials[(size_t)b * kPartialStride + q];
+		t += partials[(size_t)q * nb + b];
 	block_sum2(dummy, t);
 	if (threadIdx.x == 0)
 		marg[q] = t;
@@ -2547,8 +2572,8 @@ template <> struct FxShape<float> {
 
 template <typename R, bool NARROW>
 static cudaError_t run_sweep_fx(const void *in, void *out, const unsigned char *dprog,
-				const dk_sweep_hdr *hp, int sums, int num_sms, const Scratch &s,
-				cudaStream_t st, int *blocks_out)
+				const dk_sweep_hdr *hp, int sums, const dk_scal *sc_in, dk_scal *sc_out,
+				int num_sms, const Scratch &s, cudaStream_t st)
 {
 	typedef typename CT<R>::T C2;
 	constexpr int MINB = FxShape<R>::ctas;
@@ -2594,8 +2619,8 @@ static cudaError_t run_sweep_fx(const void *in, void *out, const unsigned char *
 	blocks = skip_balanced_grid(blocks, in, out, hp);
 	const int threads = NARROW ? 32 : 1 << (hp->m - DK_FX_BITS);
 	kern<<<(int)blocks, threads, smem, st>>>((const C2 *)in, (C2 *)out, dprog, sums,
-						 s.partials);
-	*blocks_out = (int)blocks;
+						 hp->all_touched || in != out, s.partials,
+						 (unsigned *)(s.u64 + 3), sc_in, sc_out);
 	return cudaGetLastError();
 }
 
@@ -2604,26 +2629,11 @@ cudaError_t launch_sweep_fx(int prec, const void *in, void *out, const unsigned 
 			    const Scratch &s, int num_sms, cudaStream_t st)
 {
 	g_num_sms = num_sms;
-	int blocks = 0;
 	const bool narrow = hp->m < DK_FX_BITS + 5;
-	cudaError_t e;
-	if (prec == DK_C128)
-		e = narrow ? run_sweep_fx<double, true>(in, out, dprog, hp, sums, num_sms, s, st, &blocks)
-			   : run_sweep_fx<double, false>(in, out, dprog, hp, sums, num_sms, s, st,
-							 &blocks);
-	else
-		e = narrow ? run_sweep_fx<float, true>(in, out, dprog, hp, sums, num_sms, s, st, &blocks)
-			   : run_sweep_fx<float, false>(in, out, dprog, hp, sums, num_sms, s, st,
-							&blocks);
-	if (e != cudaSuccess)
-		return e;
+	auto run = prec == DK_C128 ? (narrow ? run_sweep_fx<double, true> : run_sweep_fx<double, false>)
+				   : (narrow ? run_sweep_fx<float, true> : run_sweep_fx<float, false>);
 	g_launches += 1;
-	if (sums) {
-		const int all = hp->all_touched || (in != out);
-		k_finalize<<<1, 256, 0, st>>>(s.partials, blocks, sc_in, sc_out, FIN_GATE, all);
-		g_launches += 1;
-	}
-	return cudaGetLastError();
+	return run(in, out, dprog, hp, sums, sc_in, sc_out, num_sms, s, st);
 }
 
 cudaError_t tm_fault_check(cudaStream_t st, unsigned *faults)
@@ -2830,11 +2840,13 @@ static void launch_marginals_kernel(int prec, const void *d, unsigned n, int sbi
 cudaError_t launch_marginals(int prec, const void *d, unsigned n, const Scratch &s,
 			     cudaStream_t st)
 {
-	/* up to 2048 blocks: 2 per SM make 6.9 waves of 296 at 30 qubits */
+	/* up to 2048 blocks: 2 per SM make 6.9 waves of 296 at 30 qubits; one, whose
+	 * sums are the result, up to 12 qubits (4 us; 16 blocks and the sum over them
+	 * 4 and 3) */
 	int threads = 256, blocks = 1;
 	if (n < 8)
 		threads = 1 << n;
-	else {
+	else if (n > 12) {
 		int lb = (int)n - 8;
 		if (lb > 11)
 			lb = 11;
@@ -2850,9 +2862,13 @@ cudaError_t launch_marginals(int prec, const void *d, unsigned n, const Scratch 
 		threads = 32;
 		sbits = (int)n;
 	}
-	launch_marginals_kernel(prec, d, n, sbits, blocks, threads, s.partials, st);
-	k_marg_finalize<<<n + 1, 256, 0, st>>>(s.partials, blocks, s.marg);
-	g_launches += 2;
+	launch_marginals_kernel(prec, d, n, sbits, blocks, threads, blocks == 1 ? s.marg : s.partials,
+				st);
+	g_launches += 1;
+	if (blocks > 1) {
+		k_marg_finalize<<<n + 1, 256, 0, st>>>(s.partials, blocks, s.marg);
+		g_launches += 1;
+	}
 	return cudaGetLastError();
 }
 

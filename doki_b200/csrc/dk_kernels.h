@@ -37,7 +37,8 @@ constexpr int kPartialStride = 64;
 
 struct Scratch {
 	double *partials; /* kMaxBlocks * kPartialStride doubles */
-	unsigned long long *u64; /* 4 words */
+	unsigned long long *u64; /* 4 words: a result, measured bits, -, a count of
+				* finished blocks (0 between launches) */
 	double *marg; /* 64 doubles: marginal sums + total */
 };
 

@@ -118,6 +118,8 @@ int create_slot(int id)
 	if (e == cudaSuccess)
 		e = cudaMalloc(&sl->scratch.u64, 4 * sizeof(unsigned long long));
 	if (e == cudaSuccess)
+		e = cudaMemsetAsync(sl->scratch.u64, 0, 4 * sizeof(unsigned long long), sl->st);
+	if (e == cudaSuccess)
 		e = cudaMalloc(&sl->scratch.marg, 64 * sizeof(double));
 	if (e != cudaSuccess) {
 		snprintf(g.err, sizeof(g.err), "%s", cudaGetErrorString(e));
@@ -435,8 +437,8 @@ static int flush_queued(dk_state *s)
 	/* Factored complex64 sweeps pin 4 low qubits (128-byte runs, as complex128
 	 * sweeps pin 2 for 64-byte ones): at 28 qubits, depth 20, 36 and 34 sweeps
 	 * (brickwork, random pairs) in 59.5 and 56.7 ms against 30 and 29 sweeps in
-	 * 60.4 and 61.3 ms with 2 pinned.  complex128: 107.2 and 107.0 ms with 2,
-	 * 112.6 and 108.0 ms with 4.  A register that stays in the L2 cache (below
+	 * 60.4 and 61.3 ms with 2 pinned.  complex128: 97.2 and 97.5 ms with 2,
+	 * 101.3 and 96.9 with 3, 101.2 and 97.5 with 4.  A register that stays in the L2 cache (below
 	 * 24 qubits) gains nothing from longer runs. */
 	if (fx && prec == DK_C64 && n >= 24)
 		lim.low_bits = 4;

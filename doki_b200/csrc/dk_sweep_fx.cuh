@@ -13,10 +13,11 @@
  * What bounds it: FP64 (FP32) arithmetic and shared-memory wavefronts, about
  * half each of a sweep's time beside the streaming; they overlap little, since
  * the groups of warps that one register file holds are few.  A sweep of the
- * 28-qubit brickwork circuit takes 3.57 ms in complex128 (4.13 with 8x8 complex
+ * 28-qubit brickwork circuit takes 3.24 ms in complex128 (4.13 with 8x8 complex
  * products on FP64 MMAs) and 1.65 ms in complex64 (3.02 with TF32-split
  * products in tensor memory; 2.01 at the same number of sweeps); the streaming
- * alone takes 1.75 and 0.89.  Tried and slower: a ring of three tile buffers for
+ * alone takes 1.75 and 0.89.  Tried and slower, at 3.57 ms before the kernel made
+ * the register's scalars itself: a ring of three tile buffers for
  * two groups of one CTA, the next tile in flight throughout (4.15 ms), 11-bit
  * tiles (3.85), every stage with its four rotations whether it has them or not
  * (3.90).  Coefficients read one by one at their use instead of in batches: 3.62.
@@ -287,7 +288,8 @@ __device__ __forceinline__ void fx_sweep(const typename CT<R>::T *__restrict__ i
 		sro[tid] = (uint32_t)sizeof(C2) * swz_map(1u << (lanes + tid), h->bankv);
 		poff[tid] = (uint64_t)sizeof(C2) << h->qpos[__ffs(last->pm[tid]) - 1];
 	}
-	for (int e = tid; e < DK_DEP_NIBBLES * 16; e += blockDim.x) {
+	const int ndep = (h->n - m + 3) >> 2;
+	for (int e = tid; e < ndep * 16; e += blockDim.x) {
 		uint64_t v = (uint64_t)(e & 15) << (4 * (e >> 4));
 		for (int j = 0; j < m; ++j) {
 			const int q = h->qpos[j];
@@ -314,7 +316,6 @@ __device__ __forceinline__ void fx_sweep(const typename CT<R>::T *__restrict__ i
 	const uint32_t stid = (uint32_t)sizeof(C2) * swz_map(tid & ((1u << lanes) - 1u), h->bankv);
 	__syncthreads();
 	const uint64_t ntiles = h->ntiles;
-	const int ndep = (h->n - m + 3) >> 2;
 	const bool skip_idle = (in == out) && !h->all_touched;
 
 	auto tile_base = [&](uint64_t t) -> uint64_t {

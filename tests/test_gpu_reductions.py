@@ -18,7 +18,7 @@ def register(d, n, prec, seed):
 
 
 @pytest.mark.parametrize("prec", [2, 1])
-@pytest.mark.parametrize("n", [1, 4, 5, 7, 8, 9, 13, 17, 20])
+@pytest.mark.parametrize("n", [1, 4, 5, 7, 8, 9, 12, 13, 17, 20])
 def test_marginals_of_every_block_shape(dk_gpu, n, prec):
     """One warp with idle lanes up to the full grid.  Both sides add the same
     2^n FP64 squares in another order: within 2^n * eps at worst, far less

@@ -75,3 +75,19 @@ def test_other_sweeps_in_between(dk_gpu, orc, prec):
     for _ in range(6):
         ops += one_qubit_ops(rng, n, 20) + random_ops(rng, n, 10)
     check(dk_gpu, orc, n, prec, ops, 351)
+
+
+@pytest.mark.parametrize("prec", [2, 1])
+def test_norm_between_measurements(dk_gpu, orc, prec):
+    """The blocks of a sweep count themselves down to the last, which makes the
+    norm, in a scratch that measurements use too: flushes of 1 to 32 blocks with
+    joint measurements in between."""
+    for n in (12, 13, 17, 14):
+        rng = W.rng_for(340 + n)
+        mask = sum(1 << int(q) for q in rng.permutation(n)[:3])
+        reg = W.run_ops(dk_gpu, dk_gpu.registry_new(n, False, prec), one_qubit_ops(rng, n, 20))
+        for _ in range(3):
+            left, _ = dk_gpu.registry_measure(reg, mask, [0.3, 0.6, 0.9], -1, False)
+            assert abs(np.linalg.norm(dk_gpu.registry_get_all(left, False)) - 1) < 1e-5
+            reg = W.run_ops(dk_gpu, reg, one_qubit_ops(rng, n, 10))
+            assert abs(np.linalg.norm(dk_gpu.registry_get_all(reg, False)) - 1) < 1e-5
