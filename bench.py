@@ -62,8 +62,7 @@ def parse():
     p.add_argument("--form-only", choices=("batch", "serve", "precision"),
                    help="run only this form and print its JSON object")
     p.add_argument("--precision", choices=("c128", "c64"), default="c128",
-                   help="register precision of the plain workload (c64: split-TF32 "
-                        "tensor products, FP64 norms)")
+                   help="register precision of the plain workload (c64: FP64 norms)")
     return p.parse_args()
 
 
@@ -385,7 +384,12 @@ def engine_arm(args, rank, world, local_rank):
     e2e_value = job_rate(world, layers, e2e_s)
     c64 = args.precision == "c64"
     tcgen05 = c64 and os.environ.get("DK_C64_TMEM", "1") != "0"
-    lib_tflops = library_gemm_tflops(torch, c64) if rank == 0 and world == 1 else None
+    # factored sweeps (the default) are FMA work: no tensor pipe to account for
+    factored = os.environ.get("DK_FACTORED", "1") != "0" and not (
+        c64 and "DK_C64_TMEM" in os.environ)
+    lib_tflops = None
+    if rank == 0 and world == 1 and not factored:
+        lib_tflops = library_gemm_tflops(torch, c64)
     state_bytes = (8 if c64 else 16) << n
     avg_sweep_s = (sweep_ms / 1e3) / max(1, nsweeps)
     achieved = 2 * state_bytes / avg_sweep_s / 1e9
@@ -402,7 +406,9 @@ def engine_arm(args, rank, world, local_rank):
         "vs_baseline": None, "dtype": "f32" if c64 else "f64", "data": "synthetic",
         "config": workload_config(n, depth, c, args.precision),
         "roofline": {"bound": "hbm",
-                     "kernel": ("k_sweep_tm (fused gate sweep, split-TF32 tcgen05 products "
+                     "kernel": (f"k_sweep_fx<{'float' if c64 else 'double'}> (fused gate sweep, "
+                                "real rotations and diagonals in registers)" if factored else
+                                "k_sweep_tm (fused gate sweep, split-TF32 tcgen05 products "
                                 "in tensor memory)" if tcgen05 else
                                 "k_sweep_tc<float> (fused gate sweep, split-TF32 tensor-core "
                                 "passes)" if c64 else
@@ -417,10 +423,9 @@ def engine_arm(args, rank, world, local_rank):
         "e2e": {"value": e2e_value, "unit": UNIT,
                 "h2d_bytes_per_step": (io1["h2d_bytes"] - io0["h2d_bytes"]) // args.steps,
                 "d2h_bytes_per_step": (io1["d2h_bytes"] - io0["d2h_bytes"]) // args.steps},
-        "tensor_roofline": tensor_roofline(st1["mma_entry_amplitudes"] -
-                                           st0["mma_entry_amplitudes"],
-                                           sweep_ms / 1e3, c64, clk, args.steps,
-                                           lib_tflops, tcgen05),
+        "tensor_roofline": None if factored else
+        tensor_roofline(st1["mma_entry_amplitudes"] - st0["mma_entry_amplitudes"],
+                        sweep_ms / 1e3, c64, clk, args.steps, lib_tflops, tcgen05),
         "gpu_launches": st1["kernel_launches"] - st0["kernel_launches"],
         "clocks": clk,
         "fusion": not args.no_fusion,
@@ -430,7 +435,9 @@ def engine_arm(args, rank, world, local_rank):
     if rank == 0 and world == 1 and not args.no_forms:
         out["forms"] = run_forms(d, args, torch)
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
-        out["cpu_baseline"] = cpu_baseline(n, c)
+        from oracle import oracle as O
+        out["cpu_baseline"] = cpu_baseline(n, c) if O.have_reference() else {
+            "unavailable": "reference module not built (oracle/_ref)"}
     if world > 1:
         torch.distributed.destroy_process_group()
     if rank == 0:
