@@ -1220,16 +1220,30 @@ static void split_x(const cpx *m, cpx *rx, fx_gate *g)
 	g->s = -cdiv(w[1], cmul(w[0], r1)).x;
 }
 
+/* A factor on its way from a gate to a later one on the same qubit. */
+typedef struct fx_pending {
+	cpx w[4];
+	int from; /* the gate that gave it, -1: none on its way */
+	fx_gate whole; /* that gate with the factor in it */
+} fx_pending;
+
 /* Moves factors of uncontrolled one-qubit gates to the next such gate on the
  * same qubit, where they join its matrix: the whole gate when nothing on the
  * qubit lies in between, its left phase through gates that are diagonal on the
  * qubit (controls among them), a left Rx through X and its controlled forms.
  * What stays is k [[1, -s], [t, 1]] diag(1, r1): one product in front of the
- * rotations of a stage and none behind them. */
-static void move_factors(dk_fx_plan *P)
+ * rotations of a stage and none behind them.
+ *
+ * Roundings add up along a run of gates, so a product of matrices that have a
+ * factoring need not have one.  A factor is taken only by a gate whose product
+ * with it has one; otherwise it goes back into the gate that gave it, and every
+ * gate keeps a factoring throughout. */
+static int move_factors(dk_fx_plan *P)
 {
 	uint8_t path[64];
-	cpx pend[64][4];
+	fx_pending *pend = (fx_pending *)malloc(sizeof(*pend) * P->n);
+	if (!pend)
+		return DK_ERR_ALLOC;
 	memset(path, PUSH_NONE, sizeof(path));
 	uint8_t *push = (uint8_t *)P->order; /* nops ints: free until the first sweep */
 	for (int i = P->nops - 1; i >= 0; i--) {
@@ -1240,14 +1254,15 @@ static void move_factors(dk_fx_plan *P)
 			const unsigned q = op->tg[0];
 			uint8_t *w = &path[q];
 			if (g->kind == FX_DIAG) {
-				/* moves as a whole, or stays and is passed like a control */
+				/* moves as a whole, or stays and stops what comes before it */
 				if (g->unitary && (*w == PUSH_ALL || *w == PUSH_Z))
 					push[i] = PUSH_ALL;
 				else
 					*w = PUSH_NONE;
 				continue;
 			}
-			/* multiples of unitaries only: their products keep a factoring */
+			/* multiples of unitaries only: their products keep a factoring,
+			 * up to roundings */
 			push[i] = g->unitary ? *w : PUSH_NONE;
 			*w = g->unitary ? PUSH_ALL : PUSH_NONE;
 			continue;
@@ -1264,48 +1279,52 @@ static void move_factors(dk_fx_plan *P)
 			*w = *w == PUSH_ALL || *w == PUSH_Z ? PUSH_Z : PUSH_NONE;
 		}
 	}
-	uint64_t have = 0; /* qubits with a pending factor */
+	for (unsigned q = 0; q < P->n; q++)
+		pend[q].from = -1;
 	for (int i = 0; i < P->nops; i++) {
 		fx_gate *g = &P->g[i];
-		if (P->ops[i].k != 1 || g->ctl || (!(have >> P->ops[i].tg[0] & 1u) && !push[i]))
+		if (P->ops[i].k != 1 || g->ctl)
 			continue;
-		const unsigned q = P->ops[i].tg[0];
-		cpx m[4], *w = pend[q];
+		fx_pending *pd = &pend[P->ops[i].tg[0]];
+		if (pd->from < 0 && !push[i])
+			continue;
+		cpx m[4], *w = pd->w;
 		load1(&P->ops[i], m);
-		if (have >> q & 1u) {
+		if (pd->from >= 0) {
 			cpx t[4];
 			for (int r = 0; r < 2; r++)
 				for (int c = 0; c < 2; c++) {
 					const cpx x = cmul(m[2 * r], w[c]), y = cmul(m[2 * r + 1], w[2 + c]);
 					t[2 * r + c] = cx(x.x + y.x, x.y + y.y);
 				}
-			/* a diagonal gate that stays lets the phase of a gate before it
-			 * through (nothing else is pending there) */
-			if (g->kind == FX_DIAG && push[i] == PUSH_NONE)
-				continue;
-			memcpy(m, t, sizeof(m));
-			have &= ~tbit(q);
+			fx_gate f = *g;
+			factor1(t, &f);
+			if (f.kind != FX_NONE) {
+				*g = f;
+				memcpy(m, t, sizeof(m));
+			} else {
+				P->g[pd->from] = pd->whole;
+			}
+			pd->from = -1;
 		}
+		if (push[i] == PUSH_NONE)
+			continue;
+		pd->from = i;
+		pd->whole = *g;
 		if (push[i] == PUSH_ALL) {
 			memcpy(w, m, sizeof(m));
-			have |= tbit(q);
 			g->gone = 1;
-			continue;
-		}
-		if (push[i] == PUSH_X) {
+		} else if (push[i] == PUSH_X) {
 			split_x(m, w, g);
-			have |= tbit(q);
-			continue;
-		}
-		factor1(m, g);
-		if (push[i] == PUSH_Z) {
+		} else {
 			w[0] = c_one;
 			w[1] = w[2] = cx(0, 0);
 			w[3] = cdiv(g->l1, g->l0);
 			g->l1 = g->l0;
-			have |= tbit(q);
 		}
 	}
+	free(pend);
+	return DK_OK;
 }
 
 /* ---- the plan ------------------------------------------------------------- */
@@ -1345,8 +1364,10 @@ int dk_fx_begin(const dk_flat_op *ops, int nops, unsigned n, int prec,
 	}
 	/* gates that dk_plan.c plans from their matrices take no factor */
 	P->all = all;
-	if (all)
-		move_factors(P);
+	if (all && move_factors(P)) {
+		dk_fx_end(P);
+		return DK_ERR_ALLOC;
+	}
 	P->nops = 0;
 	for (int i = 0; i < nops; i++) {
 		fx_gate *g = &P->g[i];
@@ -1461,6 +1482,10 @@ int dk_fx_next(dk_fx_plan *P, dk_step *step, const unsigned char **prog)
 		P->head = i - nd;
 		memcpy(P->rem + P->head, defer, sizeof(int) * (size_t)nd);
 		if (!factored) {
+			/* dk_plan.c sees the gates as they were given: not for a plan
+			 * whose gates have taken factors of others */
+			if (P->all)
+				return -DK_ERR_ARG; /* cannot happen: every gate has a factoring */
 			const int rc = sub_plan(P, nt);
 			if (rc)
 				return -rc;
