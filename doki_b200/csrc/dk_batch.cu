@@ -29,6 +29,7 @@
 #include <thread>
 #include <vector>
 
+#include "dk_batch_plan.h"
 #include "dk_device.cuh"
 #include "dk_internal.h"
 #include "dk_kernels.h"
@@ -720,48 +721,11 @@ static int batch_build(int precision, unsigned num_circuits, const unsigned *num
 	 * cores: circuit c goes to worker c mod T.  Each circuit's sweep
 	 * programs are kept back to back in its own byte vector. */
 	struct Planned {
-		std::vector<unsigned char> prog;
-		uint32_t nsweep = 0, most = 0;
+		dk::BatchProgram prog;
 		int fx = 0;
 		int rc = 0;
 	};
 	std::vector<Planned> planned(num_circuits);
-	/* 0: planned (or failed with *rc), 1: some gate has no factoring */
-	auto plan_factored = [](const std::vector<dk_flat_op> &flat, unsigned n, int prec, int m,
-				std::vector<unsigned char> *prog, uint32_t *nsweep, uint32_t *most,
-				int *fx, int *rc) -> int {
-		dk_plan_limits lim = {};
-		lim.tile_bits = m;
-		dk_plan_default_limits(prec, n, &lim);
-		lim.tile_bits = m;
-		dk_fx_plan *fp = nullptr;
-		*rc = dk_fx_begin(flat.data(), (int)flat.size(), n, prec, &lim, &fp);
-		if (*rc)
-			return 0;
-		if (!dk_fx_all(fp)) {
-			dk_fx_end(fp);
-			return 1;
-		}
-		dk_step step;
-		const unsigned char *src;
-		int more;
-		while ((more = dk_fx_next(fp, &step, &src)) > 0) {
-			const uint32_t bytes = ((const dk_sweep_hdr *)src)->bytes;
-			try {
-				prog->insert(prog->end(), src, src + bytes);
-			} catch (...) {
-				more = -DK_ERR_ALLOC;
-				break;
-			}
-			++*nsweep;
-			if (bytes > *most)
-				*most = bytes;
-		}
-		dk_fx_end(fp);
-		*fx = 1;
-		*rc = more < 0 ? -more : 0;
-		return 0;
-	};
 	auto plan_some = [&](unsigned first, unsigned stride) {
 		std::vector<dk_gate> gates;
 		std::vector<dk_flat_op> flat;
@@ -801,9 +765,10 @@ static int batch_build(int precision, unsigned num_circuits, const unsigned *num
 			if (lim.low_bits > m - 3)
 				lim.low_bits = m - 3;
 			/* factored sweeps when every gate has a factoring */
-			if (!plan_factored(flat, n, precision, m, &pl.prog, &pl.nsweep, &pl.most, &pl.fx,
-					   &pl.rc))
+			if (!dk::plan_factored(flat, n, precision, m, &pl.prog, &pl.rc)) {
+				pl.fx = 1;
 				continue;
+			}
 			dk_plan plan;
 			pl.rc = dk_plan_build(flat.data(), (int)flat.size(), n, precision, &lim, &plan);
 			if (pl.rc)
@@ -815,26 +780,26 @@ static int batch_build(int precision, unsigned num_circuits, const unsigned *num
 				}
 				const dk_sweep_hdr *h =
 					(const dk_sweep_hdr *)(plan.blob + plan.steps[st].prog_off);
-				const size_t at = pl.prog.size();
+				const size_t at = pl.prog.bytes.size();
 				try {
-					pl.prog.resize(at + h->bytes);
+					pl.prog.bytes.resize(at + h->bytes);
 				} catch (...) {
 					pl.rc = DK_ERR_ALLOC;
 					break;
 				}
-				memcpy(pl.prog.data() + at, h, h->bytes);
+				memcpy(pl.prog.bytes.data() + at, h, h->bytes);
 				if (precision == DK_C64) {
 					/* store the matrices in the amplitude precision, in place */
-					dk_sweep_hdr *hh = (dk_sweep_hdr *)(pl.prog.data() + at);
+					dk_sweep_hdr *hh = (dk_sweep_hdr *)(pl.prog.bytes.data() + at);
 					const double *src =
-						(const double *)(pl.prog.data() + at + hh->mat_off);
-					float *dst = (float *)(pl.prog.data() + at + hh->mat_off);
+						(const double *)(pl.prog.bytes.data() + at + hh->mat_off);
+					float *dst = (float *)(pl.prog.bytes.data() + at + hh->mat_off);
 					const size_t nv = 2 * ((hh->bytes - hh->mat_off) / 16);
 					for (size_t v = 0; v < nv; ++v)
 						dst[v] = (float)src[v];
 				}
 			}
-			pl.nsweep = (uint32_t)plan.nsteps;
+			pl.prog.nsweep = (uint32_t)plan.nsteps;
 			dk_plan_free(&plan);
 		}
 	};
@@ -863,7 +828,7 @@ static int batch_build(int precision, unsigned num_circuits, const unsigned *num
 	for (unsigned c = 0; c < num_circuits; ++c) {
 		const size_t pad = ((blob_len + 15) & ~(size_t)15) - blob_len;
 		at[c] = blob_len + pad;
-		blob_len = at[c] + planned[c].prog.size();
+		blob_len = at[c] + planned[c].prog.bytes.size();
 	}
 	blob.reset(new (std::nothrow) unsigned char[blob_len ? blob_len : 16]);
 	if (!blob) {
@@ -873,10 +838,10 @@ static int batch_build(int precision, unsigned num_circuits, const unsigned *num
 	{
 		auto copy_some = [&](unsigned first, unsigned stride) {
 			for (unsigned c = first; c < num_circuits; c += stride) {
-				if (!planned[c].prog.empty())
-					memcpy(blob.get() + at[c], planned[c].prog.data(),
-					       planned[c].prog.size());
-				std::vector<unsigned char>().swap(planned[c].prog);
+				if (!planned[c].prog.bytes.empty())
+					memcpy(blob.get() + at[c], planned[c].prog.bytes.data(),
+					       planned[c].prog.bytes.size());
+				std::vector<unsigned char>().swap(planned[c].prog.bytes);
 			}
 		};
 		run_strided(T, copy_some);
@@ -888,7 +853,7 @@ static int batch_build(int precision, unsigned num_circuits, const unsigned *num
 		dk_breg reg;
 		memset(&reg, 0, sizeof(reg));
 		reg.prog = at[c];
-		reg.nsweep = planned[c].nsweep;
+		reg.nsweep = planned[c].prog.nsweep;
 		reg.n = n;
 		reg.keep = keep;
 		reg.state = b->state_amps;
@@ -910,8 +875,8 @@ static int batch_build(int precision, unsigned num_circuits, const unsigned *num
 		}
 		BatchClass &cl = b->classes[class_of[key]];
 		cl.regs.push_back(reg);
-		if (planned[c].most > cl.most)
-			cl.most = planned[c].most;
+		if (planned[c].prog.most > cl.most)
+			cl.most = planned[c].prog.most;
 	}
 	/* larger registers and longer circuits first, in a class and among the
 	 * classes (better tail balance) */
