@@ -370,31 +370,33 @@ __global__ void __launch_bounds__(kFxThreads, MINB)
 				/* no tile conditions: one list */
 				const uint4 ph = __ldg(reinterpret_cast<const uint4 *>(pd));
 				const uint4 l0 = __ldg(lists + 2 * ph.y), l1 = __ldg(lists + 2 * ph.y + 1);
-				if (l1.w && !(ph.x & DK_FX_STORE))
-					continue;
-				const uint32_t sg = __ldg(&pd->slo[lane]) ^ __ldg(&pd->shi[warp]);
-				C2 a[DK_FX_REGS];
-				auto slot = [&](int q, uint32_t base, uint32_t x, uint32_t y) -> uint32_t {
-					return base ^ ((q & 1) ? x & 0xffffu : 0u) ^ ((q & 2) ? x >> 16 : 0u) ^
-					       ((q & 4) ? y & 0xffffu : 0u) ^ ((q & 8) ? y >> 16 : 0u);
-				};
-				const uint32_t gb = sg ^ (l1.x & 0xffffu), sb = sg ^ (l1.x >> 16);
+				/* a pass with nothing to do ends with its barrier all the same: the
+				 * last of a phase separates warps that the others do not */
+				if (!l1.w || (ph.x & DK_FX_STORE)) {
+					const uint32_t sg = __ldg(&pd->slo[lane]) ^ __ldg(&pd->shi[warp]);
+					C2 a[DK_FX_REGS];
+					auto slot = [&](int q, uint32_t base, uint32_t x, uint32_t y) -> uint32_t {
+						return base ^ ((q & 1) ? x & 0xffffu : 0u) ^ ((q & 2) ? x >> 16 : 0u) ^
+						       ((q & 4) ? y & 0xffffu : 0u) ^ ((q & 8) ? y >> 16 : 0u);
+					};
+					const uint32_t gb = sg ^ (l1.x & 0xffffu), sb = sg ^ (l1.x >> 16);
 #pragma unroll
-				for (int q = 0; q < DK_FX_REGS; ++q)
-					a[q] = *reinterpret_cast<const C2 *>(tile + slot(q, gb, l0.x, l0.y));
-				const uint32_t raw = (ph.x & DK_PASS_CTL)
-							     ? (__ldg(&pd->rlo[lane]) | __ldg(&pd->rhi[warp]))
-							     : 0u;
-				const uint32_t o1 = l1.y >> 16;
-				for (uint32_t o = l1.y & 0xffffu; o < o1; ++o) {
-					const uint4 d = __ldg(ops + o);
-					if ((d.z | d.w) && !ctl_ok(raw, d.z, d.w))
-						continue;
-					fx_op<true>(a, d.x & 0xffffu, d.x >> 16, table + d.y);
+					for (int q = 0; q < DK_FX_REGS; ++q)
+						a[q] = *reinterpret_cast<const C2 *>(tile + slot(q, gb, l0.x, l0.y));
+					const uint32_t raw = (ph.x & DK_PASS_CTL)
+								     ? (__ldg(&pd->rlo[lane]) | __ldg(&pd->rhi[warp]))
+								     : 0u;
+					const uint32_t o1 = l1.y >> 16;
+					for (uint32_t o = l1.y & 0xffffu; o < o1; ++o) {
+						const uint4 d = __ldg(ops + o);
+						if ((d.z | d.w) && !ctl_ok(raw, d.z, d.w))
+							continue;
+						fx_op<true>(a, d.x & 0xffffu, d.x >> 16, table + d.y);
+					}
+#pragma unroll
+					for (int q = 0; q < DK_FX_REGS; ++q)
+						*reinterpret_cast<C2 *>(tile + slot(q, sb, l0.z, l0.w)) = a[q];
 				}
-#pragma unroll
-				for (int q = 0; q < DK_FX_REGS; ++q)
-					*reinterpret_cast<C2 *>(tile + slot(q, sb, l0.z, l0.w)) = a[q];
 				if ((ph.x & DK_PASS_WARP) && G >= 64)
 					__syncwarp();
 				else
