@@ -24,8 +24,12 @@
 
 #include "dk_internal.h"
 #include "dk_kernels.h"
+#include "dk_stage_ring.h"
 
 namespace {
+
+constexpr size_t kStagePart = 1u << 20;
+constexpr int kStageParts = 2;
 
 /* A slot: one CUDA stream with its own scratch and lock.  Every
  * register belongs to the slot that created it (derived registers inherit
@@ -42,13 +46,9 @@ struct Slot {
 	 * the device side needs no wait, since copies and sweeps share the
 	 * slot's stream.  Allocated by the slot's first flush, kept with it. */
 	unsigned char *stage_host = nullptr, *stage_dev = nullptr;
-	size_t stage_at = 0;
-	cudaEvent_t copied[2] = { nullptr, nullptr };
-	bool in_use[2] = { false, false };
+	dk::StageRing<kStagePart, kStageParts> stage;
+	cudaEvent_t copied[kStageParts] = {};
 };
-
-constexpr size_t kStagePart = 1u << 20;
-constexpr int kStageParts = 2;
 
 constexpr int kMaxSlots = 64;
 
@@ -315,23 +315,24 @@ static int stage_up(const void *src, size_t bytes, const unsigned char **dev, vo
 			CK(cudaMalloc(&sl.stage_dev, kStagePart * kStageParts));
 		CK(cudaHostAlloc(&sl.stage_host, kStagePart * kStageParts, cudaHostAllocDefault));
 	}
-	int part = (int)(sl.stage_at / kStagePart);
-	if (sl.stage_at + bytes > (size_t)(part + 1) * kStagePart) {
-		/* the next part: its last copies must have left the host buffer */
-		CK(cudaEventRecord(sl.copied[part], sl.st));
-		sl.in_use[part] = true;
-		part = (part + 1) % kStageParts;
-		sl.stage_at = (size_t)part * kStagePart;
-		if (sl.in_use[part])
+	size_t at;
+	const int rc = sl.stage.place(
+		bytes,
+		[&](int part) -> int {
+			CK(cudaEventRecord(sl.copied[part], sl.st));
+			return DK_OK;
+		},
+		[&](int part) -> int {
 			CK(cudaEventSynchronize(sl.copied[part]));
-	}
-	memcpy(sl.stage_host + sl.stage_at, src, bytes);
-	CK(cudaMemcpyAsync(sl.stage_dev + sl.stage_at, sl.stage_host + sl.stage_at, bytes,
-			   cudaMemcpyHostToDevice, sl.st));
-	*dev = sl.stage_dev + sl.stage_at;
-	sl.stage_at += (bytes + 255) & ~(size_t)255;
-	if (sl.stage_at >= kStagePart * kStageParts)
-		sl.stage_at = kStagePart * kStageParts - 1; /* full: the next call moves on */
+			return DK_OK;
+		},
+		&at);
+	if (rc)
+		return rc;
+	memcpy(sl.stage_host + at, src, bytes);
+	CK(cudaMemcpyAsync(sl.stage_dev + at, sl.stage_host + at, bytes, cudaMemcpyHostToDevice,
+			   sl.st));
+	*dev = sl.stage_dev + at;
 	return DK_OK;
 }
 
