@@ -28,8 +28,7 @@ NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
 CU_SOURCES = ["dk_kernels.cu", "dk_runtime.cu", "dk_noalloc.cu", "dk_batch.cu"]
 C_SOURCES = ["dk_plan.c", "dk_plan_fx.c"]
 HEADERS = ["dk_internal.h", "dk_kernels.h", "dk_device.cuh", "dk_sweep_fx.cuh",
-           "dk_rho_int8.cuh", "dk_batch_plan.h",
-           "dk_stage_ring.h"]
+           "dk_batch_plan.h", "dk_stage_ring.h"]
 
 LIB = os.path.join(HERE, "libdokigpu.so")
 # Debug build: the kernels check every index they compute

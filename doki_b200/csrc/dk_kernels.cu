@@ -11,7 +11,6 @@
 #include <stdint.h>
 #include <string.h>
 
-#include <algorithm>
 #include <mutex>
 
 #include "dk_device.cuh"
@@ -2058,6 +2057,8 @@ __global__ void __launch_bounds__(256)
 	}
 }
 
+/* The whole matrix from its lower triangle.  A sum of |x|^2 has no imaginary part:
+ * what the products' roundings left of it on the diagonal goes (a NaN stays). */
 __global__ void __launch_bounds__(256)
 	k_herm_fill(const double2 *__restrict__ C, double2 *rho, uint64_t dim)
 {
@@ -2066,9 +2067,12 @@ __global__ void __launch_bounds__(256)
 	     e += (uint64_t)gridDim.x * blockDim.x) {
 		const uint64_t a = e / dim, a2 = e % dim;
 		double2 v;
-		if (a >= a2)
+		if (a > a2)
 			v = C[a + a2 * dim];
-		else {
+		else if (a == a2) {
+			v = C[a + a * dim];
+			v.y -= v.y;
+		} else {
 			v = C[a2 + a * dim];
 			v.y = -v.y;
 		}
@@ -2277,8 +2281,6 @@ __global__ void __launch_bounds__(128)
 		C[e] = make_double2(alpha * x, alpha * y);
 	}
 }
-
-#include "dk_rho_int8.cuh"
 
 template <typename R>
 __global__ void __launch_bounds__(256)
@@ -3222,127 +3224,6 @@ cudaError_t launch_rho(const double2 *A, uint64_t dim, uint64_t K, double alpha,
 		k_rho_reduce<<<blocks, 128, 0, st>>>(part, nsplit, dim, alpha, C);
 		g_launches += 1;
 	}
-	return cudaGetLastError();
-}
-
-/* Chunks of the traced index for the integer products: as rho_splits, in stages
- * of kR8K traced values (2 us), with the chunk's own bound. */
-static uint64_t rho8_chunk(uint64_t dim, uint64_t K, int num_sms)
-{
-	const uint64_t T = dim / kR8Rows, tiles = 2 * T * (T + 1);
-	uint64_t best = kR8Chunk, best_cost = ~0ull;
-	for (uint64_t chunk = K < kR8Chunk ? K : kR8Chunk; chunk >= 256; chunk -= kR8K) {
-		const uint64_t ns = (K + chunk - 1) / chunk;
-		const uint64_t cost = (tiles * ns + num_sms - 1) / num_sms * (chunk / kR8K + 4) +
-				      ns * dim * dim * 32 / (13u << 20);
-		if (cost < best_cost) {
-			best = chunk;
-			best_cost = cost;
-		}
-	}
-	return best;
-}
-
-/* Integer or FP64 products: the integer ones from 2^29 complex products
- * on (and at least 1024 traced values, 128 kept ones: whole blocks).
- * Read by the host, us, integer / FP64: 7 of 21 qubits 143 / 138, 7 of 22 166 /
- * 191; 8 of 20 264 / 267, 8 of 21 277 / 304; 9 of 19 729 / 691, 9 of 21 755 /
- * 784; 10 of 20 2442 / 2495; 9 of 26 2235 / 4950. */
-bool rho_int8_plan(int prec, unsigned n, int k, int num_sms, RhoInt8 *r)
-{
-	if (prec != DK_C64 || k < 7 || n < (unsigned)k + 10 || n + (unsigned)k < 29)
-		return false;
-	const uint64_t dim = 1ull << k, K = 1ull << (n - k);
-	r->chunk = rho8_chunk(dim, K, num_sms > 0 ? num_sms : 1);
-	r->splits = (int)((K + r->chunk - 1) / r->chunk);
-	r->block_bytes = (size_t)kR8Planes << n;
-	r->part_bytes = 16 * dim * dim * (size_t)r->splits;
-	r->row_bytes = 4 * (dim + 1);
-	return r->part_bytes <= (1ull << 30);
-}
-
-cudaError_t launch_rho_int8(const void *d, unsigned n, uint64_t keep_mask, const RhoInt8 &r,
-			    void *blocks, uint32_t *rows, double2 *part, double alpha, double2 *C,
-			    int num_sms, cudaStream_t st)
-{
-	static std::once_flag once;
-	static cudaError_t set_err = cudaSuccess;
-	std::call_once(once, [] {
-		set_err = cudaFuncSetAttribute(k_rho_int8, cudaFuncAttributeMaxDynamicSharedMemorySize,
-					       2 * kR8Stage);
-	});
-	if (set_err != cudaSuccess)
-		return set_err;
-	/* register bits of the kept and traced indices, their offsets in the blocks */
-	uint64_t off[64], in_tile = 0;
-	uint32_t kept[64];
-	uint8_t by_out[64]; /* register bits, kept in order, then traced in order */
-	int k = 0, t = 0;
-	for (unsigned q = 0; q < n; ++q)
-		k += (int)((keep_mask >> q) & 1ull);
-	const uint64_t K = 1ull << (n - k), dim = 1ull << k;
-	const uint64_t row_block = K / kR8K * kR8Block;
-	k = 0;
-	for (unsigned q = 0; q < n; ++q) {
-		kept[q] = 0;
-		if ((keep_mask >> q) & 1ull) {
-			off[q] = k < 3 ? 16ull << k : k < 7 ? 512ull << (k - 3) : row_block << (k - 7);
-			kept[q] = 1u << k;
-			if (k < 3)
-				in_tile |= 1ull << q;
-			++k;
-		} else {
-			off[q] = t < 4 ? 1ull << t : t < 6 ? 128ull << (t - 4) : (uint64_t)kR8Block << (t - 6);
-			if (t < 4)
-				in_tile |= 1ull << q;
-			++t;
-		}
-	}
-	in_tile |= 31u;
-	for (unsigned q = 0; __builtin_popcountll(in_tile) < kR8TileBits; ++q)
-		in_tile |= 1ull << q;
-	R8Map map;
-	memset(&map, 0, sizeof(map));
-	int nt = 0;
-	for (unsigned q = 0; q < n; ++q)
-		if ((in_tile >> q) & 1ull)
-			by_out[nt++] = (uint8_t)q;
-	std::sort(by_out, by_out + nt, [&](uint8_t x, uint8_t y) { return off[x] < off[y]; });
-	for (int j = 0; j < nt; ++j) {
-		const unsigned q = by_out[j];
-		const int pos = __builtin_popcountll(in_tile & ((1ull << q) - 1ull));
-		map.out[j] = off[q];
-		map.kept[j] = kept[q];
-		map.in[pos] = 1ull << q;
-		map.slot[pos] = (uint16_t)r8_slot(1u << j);
-		if (kept[q])
-			map.arank[pos] = (uint16_t)(1u << map.nkept++);
-	}
-	for (int side = 0; side < 2; ++side)
-		for (unsigned q = 0; q < n; ++q)
-			if (!((in_tile >> q) & 1ull) && (kept[q] != 0) == (side == 1)) {
-				map.rin[map.rest] = 1ull << q;
-				map.rout[map.rest] = off[q];
-				map.rkept[map.rest++] = kept[q];
-				map.ntraced += side == 0;
-			}
-	const uint64_t ntiles = 1ull << map.rest;
-	cudaError_t e = cudaMemsetAsync(rows, 0, r.row_bytes, st);
-	if (e != cudaSuccess)
-		return e;
-	uint64_t per_cta = 1ull << map.ntraced;
-	while (per_cta > 1 && ntiles / per_cta < (uint64_t)num_sms * 2)
-		per_cta >>= 1;
-	k_rho_rowmax<<<(unsigned)(ntiles / per_cta), 256, 0, st>>>((const float2 *)d, map, per_cta, rows);
-	k_rho_digits<<<grid_for(ntiles, 1, num_sms * 6), 256, 0, st>>>(
-		(const float2 *)d, map, ntiles, rows, (unsigned char *)blocks);
-	const uint64_t T = dim / kR8Rows;
-	k_rho_int8<<<dim3((unsigned)(2 * T * (T + 1)), (unsigned)r.splits), kR8Threads, 2 * kR8Stage,
-		     st>>>((const unsigned char *)blocks, (uint32_t)dim, (uint32_t)K, (uint32_t)r.chunk,
-			   rows, part, rows + dim);
-	k_rho_reduce<<<grid_for(dim * dim, 128, num_sms * 16), 128, 0, st>>>(part, r.splits, dim, alpha,
-									    C);
-	g_launches += 4;
 	return cudaGetLastError();
 }
 

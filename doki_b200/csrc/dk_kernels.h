@@ -133,19 +133,6 @@ int rho_splits(uint64_t dim, uint64_t K, int num_sms);
 cudaError_t launch_rho(const double2 *A, uint64_t dim, uint64_t K, double alpha, int nsplit,
 		       double2 *part, double2 *C, cudaStream_t st);
 
-/* The same for large complex64 registers, on the integer tensor cores straight
- * from the register; rows holds dim largest components, then a count of waits that
- * expired (non-zero: the result is void). */
-struct RhoInt8 {
-	uint64_t chunk;
-	int splits;
-	size_t block_bytes, part_bytes, row_bytes;
-};
-bool rho_int8_plan(int prec, unsigned n, int k, int num_sms, RhoInt8 *r);
-cudaError_t launch_rho_int8(const void *d, unsigned n, uint64_t keep_mask, const RhoInt8 &r,
-			    void *blocks, uint32_t *rows, double2 *part, double alpha, double2 *C,
-			    int num_sms, cudaStream_t st);
-
 /* lower triangle of the column-major Hermitian C -> full row-major rho */
 cudaError_t launch_herm_fill(const double2 *C, double2 *rho, uint64_t dim,
 			     cudaStream_t st);

@@ -1656,43 +1656,26 @@ int dk_reduced_density(dk_state *s, uint64_t keep_mask, double *out)
 	const uint64_t dim = 1ull << k;
 	const uint64_t K = 1ull << (n - k);
 	const double alpha = 1.0 / (s->norm * s->norm);
-	/* integer products straight from a large complex64 register; else FP64 tensor
-	 * products X X^H of the register or of X gathered from it.  Both split the
-	 * traced index into partials that are added in a fixed order. */
-	dk::RhoInt8 r8;
-	const bool int8 = dk::rho_int8_plan(s->prec, n, k, g.num_sms, &r8);
+	/* FP64 tensor products X X^H of the register or of X gathered from it, split
+	 * over the traced index into partials that are added in a fixed order */
 	const bool direct = (s->prec == DK_C128) && (keep_mask == dim - 1);
 	const int ns = dk::rho_splits(dim, K, g.num_sms);
-	/* C, rho, X or the digit blocks, partials, row scales */
-	const size_t bytes[5] = { 16 * dim * dim, 16 * dim * dim,
-				  int8 ? r8.block_bytes : direct ? 0 : 16ull << n,
-				  int8 ? r8.part_bytes
-				       : (ns > 1 || dim < 64) ? 16 * dim * dim * (size_t)ns : 0,
-				  int8 ? r8.row_bytes : 0 };
-	void *p[5] = {};
-	for (int i = 0; i < 5 && rc == DK_OK; ++i)
+	/* C, rho, X, partials */
+	const size_t bytes[4] = { 16 * dim * dim, 16 * dim * dim, direct ? 0 : 16ull << n,
+				  (ns > 1 || dim < 64) ? 16 * dim * dim * (size_t)ns : 0 };
+	void *p[4] = {};
+	for (int i = 0; i < 4 && rc == DK_OK; ++i)
 		if (bytes[i])
 			rc = dev_alloc(&p[i], bytes[i]);
 	cudaError_t e = cudaSuccess;
-	uint32_t faults = 0;
 	if (rc == DK_OK) {
 		double2 *const C = (double2 *)p[0], *const rho = (double2 *)p[1];
-		double2 *const part = (double2 *)p[3];
-		if (int8) {
-			uint32_t *rows = (uint32_t *)p[4];
-			e = dk::launch_rho_int8(s->buf->d, n, keep_mask, r8, p[2], rows, part, alpha, C,
-						g.num_sms, CUR.st);
-			if (e == cudaSuccess)
-				e = cudaMemcpyAsync(&faults, rows + dim, sizeof(faults),
-						    cudaMemcpyDeviceToHost, CUR.st);
-		} else {
-			if (!direct)
-				e = dk::launch_gather_kept(s->prec, s->buf->d, n, keep_mask, (double2 *)p[2],
-							   CUR.st);
-			if (e == cudaSuccess)
-				e = dk::launch_rho(direct ? (const double2 *)s->buf->d : (double2 *)p[2],
-						   dim, K, alpha, ns, part, C, CUR.st);
-		}
+		if (!direct)
+			e = dk::launch_gather_kept(s->prec, s->buf->d, n, keep_mask, (double2 *)p[2],
+						   CUR.st);
+		if (e == cudaSuccess)
+			e = dk::launch_rho(direct ? (const double2 *)s->buf->d : (double2 *)p[2], dim, K,
+					   alpha, ns, (double2 *)p[3], C, CUR.st);
 		if (e == cudaSuccess)
 			e = dk::launch_herm_fill(C, rho, dim, CUR.st);
 		if (e == cudaSuccess)
@@ -1701,17 +1684,13 @@ int dk_reduced_density(dk_state *s, uint64_t keep_mask, double *out)
 		if (e == cudaSuccess)
 			e = cudaStreamSynchronize(CUR.st);
 	}
-	for (int i = 0; i < 5; ++i)
+	for (int i = 0; i < 4; ++i)
 		if (p[i])
 			dev_free(p[i], bytes[i]);
 	if (rc)
 		return rc;
 	if (e != cudaSuccess)
 		return cuda_fail(e);
-	if (faults) {
-		snprintf(g.err, sizeof(g.err), "reduced density: %u bounded waits expired", faults);
-		return DK_ERR_TIMEOUT;
-	}
 	return DK_OK;
 }
 
