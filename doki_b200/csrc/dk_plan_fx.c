@@ -207,6 +207,7 @@ struct dk_fx_plan {
 	int ngone; /* gates absorbed by others, not yet counted in a step */
 	int all; /* every gate has a factoring */
 	dk_plan_limits lim;
+	int low; /* qubits always in the tile of a factored sweep */
 	int *rem, head; /* gates left: rem[head .. nops) */
 	int *take, *order, *win; /* a sweep's gates; in pass order; a pass's leftovers */
 	dk_fx_pass *pass;
@@ -1340,6 +1341,7 @@ int dk_fx_begin(const dk_flat_op *ops, int nops, unsigned n, int prec,
 	P->n = n;
 	P->prec = prec;
 	P->lim = *lim;
+	P->low = lim->low_bits;
 	P->cpass = DK_MAX_FX_PASSES;
 	const size_t cnt = (size_t)(nops > 0 ? nops : 1);
 	P->g = (fx_gate *)calloc(cnt, sizeof(fx_gate));
@@ -1387,6 +1389,8 @@ int dk_fx_begin(const dk_flat_op *ops, int nops, unsigned n, int prec,
 
 int dk_fx_all(const dk_fx_plan *P) { return P->all; }
 
+void dk_fx_set_low_bits(dk_fx_plan *P, int low) { P->low = low; }
+
 void dk_fx_end(dk_fx_plan *P)
 {
 	if (!P)
@@ -1428,6 +1432,47 @@ static int sub_plan(dk_fx_plan *P, int cnt)
 	return rc;
 }
 
+/* A sweep's gates. */
+typedef struct fx_choice {
+	uint64_t Q; /* their targets and the pinned low qubits */
+	int nt, nd, end; /* P->take, P->order (passed over), the first not looked at */
+	int factored;
+} fx_choice;
+
+static fx_choice choose(dk_fx_plan *P, int low)
+{
+	const int m = P->lim.tile_bits;
+	if (low > m - DK_SWEEP_MAX_K)
+		low = m - DK_SWEEP_MAX_K;
+	uint64_t Q = (UINT64_C(1) << (low > 0 ? low : 0)) - 1u, blocked = 0;
+	const uint64_t full = P->n >= 64 ? ~UINT64_C(0) : (UINT64_C(1) << P->n) - 1u;
+	int nt = 0, nd = 0, factored = m >= DK_FX_MIN_TILE, i;
+	int *defer = P->order; /* free until the sweep is emitted */
+	for (i = P->head; i < P->nops && blocked != full && nt < DK_FX_MAX_GATES; i++) {
+		const int id = P->rem[i];
+		const fx_gate *g = &P->g[id];
+		const uint64_t nq = Q | g->tmask;
+		/* a gate that no sweep runs goes to dk_plan.c by itself */
+		const int sweepable = P->ops[id].k <= DK_SWEEP_MAX_K && m >= DK_PASS_BITS;
+		if (!sweepable && nt == 0 && nd == 0) {
+			P->take[nt++] = id;
+			factored = 0;
+			i++;
+			break;
+		}
+		if (sweepable && !(g->sup & blocked) && popc(nq) <= m) {
+			Q = nq;
+			P->take[nt++] = id;
+			factored &= g->kind != FX_NONE;
+		} else {
+			defer[nd++] = id;
+			blocked |= g->sup;
+		}
+	}
+	const fx_choice c = { Q, nt, nd, i, factored };
+	return c;
+}
+
 int dk_fx_next(dk_fx_plan *P, dk_step *step, const unsigned char **prog)
 {
 	const int m = P->lim.tile_bits;
@@ -1449,51 +1494,26 @@ int dk_fx_next(dk_fx_plan *P, dk_step *step, const unsigned char **prog)
 		}
 		if (P->head >= P->nops)
 			return 0;
-		/* select the next sweep's gates */
-		int low = P->lim.low_bits;
-		if (low > m - DK_SWEEP_MAX_K)
-			low = m - DK_SWEEP_MAX_K;
-		uint64_t Q = (UINT64_C(1) << (low > 0 ? low : 0)) - 1u, blocked = 0;
-		const uint64_t full = P->n >= 64 ? ~UINT64_C(0) : (UINT64_C(1) << P->n) - 1u;
-		int nt = 0, nd = 0, factored = m >= DK_FX_MIN_TILE, i;
-		int *defer = P->order; /* free until the sweep is emitted */
-		for (i = P->head; i < P->nops && blocked != full && nt < DK_FX_MAX_GATES; i++) {
-			const int id = P->rem[i];
-			const fx_gate *g = &P->g[id];
-			const uint64_t nq = Q | g->tmask;
-			/* a gate that no sweep runs goes to dk_plan.c by itself */
-			const int sweepable = P->ops[id].k <= DK_SWEEP_MAX_K && m >= DK_PASS_BITS;
-			if (!sweepable && nt == 0 && nd == 0) {
-				P->take[nt++] = id;
-				factored = 0;
-				i++;
-				break;
-			}
-			if (sweepable && !(g->sup & blocked) && popc(nq) <= m) {
-				Q = nq;
-				P->take[nt++] = id;
-				factored &= g->kind != FX_NONE;
-			} else {
-				defer[nd++] = id;
-				blocked |= g->sup;
-			}
-		}
+		fx_choice c = choose(P, P->low);
+		/* the pinned low qubits are those of the sweep that will run */
+		if (!c.factored && P->low != P->lim.low_bits)
+			c = choose(P, P->lim.low_bits);
 		/* what was passed over comes right before what was not looked at */
-		P->head = i - nd;
-		memcpy(P->rem + P->head, defer, sizeof(int) * (size_t)nd);
-		if (!factored) {
+		P->head = c.end - c.nd;
+		memcpy(P->rem + P->head, P->order, sizeof(int) * (size_t)c.nd);
+		if (!c.factored) {
 			/* dk_plan.c sees the gates as they were given: not for a plan
 			 * whose gates have taken factors of others */
 			if (P->all)
 				return -DK_ERR_ARG; /* cannot happen: every gate has a factoring */
-			const int rc = sub_plan(P, nt);
+			const int rc = sub_plan(P, c.nt);
 			if (rc)
 				return -rc;
 			continue;
 		}
-		for (unsigned q = 0; popc(Q) < m && q < P->n; q++)
-			Q |= tbit(q);
-		const int rc = emit(P, nt, Q, m, step, prog);
+		for (unsigned q = 0; popc(c.Q) < m && q < P->n; q++)
+			c.Q |= tbit(q);
+		const int rc = emit(P, c.nt, c.Q, m, step, prog);
 		return rc ? -rc : 1;
 	}
 }
