@@ -73,6 +73,7 @@ typedef struct fx_gate {
 	uint64_t sup, tmask, ctl;
 	int kind, flip;
 	int unitary, is_x; /* one qubit: a multiple of a unitary; exactly X */
+	int known; /* the factors below are those of its matrix */
 	int gone; /* absorbed by a later gate */
 	cpx l0, l1, r1;
 	real s, t;
@@ -85,14 +86,21 @@ static int popc(uint64_t x) { return __builtin_popcountll(x); }
 
 static real cabs2(cpx a) { return a.x * a.x + a.y * a.y; }
 
-/* a, b, c, d (a, d not zero) as diag(a, l1) [[1, -s], [t, 1]] diag(1, r1);
+/* What a factoring may leave out of a matrix, next to entries of size 1: the
+ * roundings of the entries of a U3 leave up to 1.6e-15. */
+#define FX_DROP 4e-15L
+
+/* a, b, c, d (a, d not zero) as diag(l0, l1) [[1, -s], [t, 1]] diag(1, r1);
  * 0 when s is not real.  r1 is a phase, so the factors stay as large as the
  * matrix.  s is real for every multiple of a unitary, up to the roundings of its
  * entries (products of several matrices among them, next to entries of size
- * 1); for other matrices it has to be real to a few roundings of itself. */
+ * 1); for other matrices it has to be real to a few roundings of itself.  The
+ * phase of b c / (a d) that keeps s from being real is left out of all four
+ * entries, in shares that leave the least error: a quarter of it from each where
+ * they are alike, half from b and c where they are small. */
 static int factor2(cpx a, cpx b, cpx c, cpx d, fx_gate *g)
 {
-	cpx r1 = c_one;
+	cpx r1 = c_one, l0 = a, l1 = d;
 	real s = 0, t = 0;
 	if (!czero(c)) {
 		const cpx w = cdiv(c, d);
@@ -103,9 +111,18 @@ static int factor2(cpx a, cpx b, cpx c, cpx d, fx_gate *g)
 		if (!czero(b)) {
 			const cpx v = cmul(cdiv(b, a), cx(r1.x, -r1.y));
 			s = -v.x;
-			if (!(fabsl(v.y) <= (g->unitary ? 1e-13L : 4e-15L * fabsl(s))) ||
+			if (!(fabsl(v.y) <= (g->unitary ? FX_DROP : FX_DROP * fabsl(s))) ||
 			    fabsl(s) > 1e6L)
 				return 0;
+			if (fabsl(v.y) <= 1e-8L * fabsl(s)) {
+				/* v = -s exp(i e): e / 2 to r1; a and d turn by e / 2 times
+				 * the part of b c in b c + a d */
+				const real x = fabsl(s) * t, e = v.y / v.x;
+				const cpx f = cx(1, e * x / (2 * (1 + x)));
+				r1 = cmul(r1, cx(1, e / 2));
+				l0 = cmul(a, f);
+				l1 = cmul(d, f);
+			}
 		}
 	} else if (!czero(b)) {
 		const cpx v = cdiv(b, a);
@@ -114,8 +131,8 @@ static int factor2(cpx a, cpx b, cpx c, cpx d, fx_gate *g)
 			return 0;
 		r1 = cx(-v.x / s, -v.y / s);
 	}
-	g->l0 = a;
-	g->l1 = cmul(d, cx(r1.x, -r1.y));
+	g->l0 = l0;
+	g->l1 = cmul(l1, cx(r1.x, -r1.y));
 	g->r1 = r1;
 	g->s = s;
 	g->t = t;
@@ -149,6 +166,31 @@ static void factor1(const cpx *m, fx_gate *g)
 		g->kind = FX_ROT;
 }
 
+/* The kind of a one-qubit matrix; its factors too unless it is a rotation of a
+ * unitary, whose factors (three divisions and a root) wait until the gate's last
+ * matrix is known.  Its s is told real from b c / (a d) with half of factor2's
+ * margin. */
+static void classify1(const cpx *m, fx_gate *g)
+{
+	if (!g->unitary || czero(m[0]) || czero(m[1]) || czero(m[2]) || czero(m[3])) {
+		factor1(m, g);
+		g->known = 1;
+		return;
+	}
+	const real na = cabs2(m[0]), nb = cabs2(m[1]), nc = cabs2(m[2]), nd = cabs2(m[3]);
+	const cpx bc = cmul(m[1], m[2]), ad = cmul(m[0], m[3]);
+	const real y = bc.y * ad.x - bc.x * ad.y;
+	g->flip = nb * nc > na * nd;
+	/* |Im s| = |y| / (|a|^2 |c| |d|), b for a and so on after an X */
+	const real f = FX_DROP / 2 * (g->flip ? nb : na);
+	g->kind = y * y <= f * f * nc * nd ? FX_ROT : FX_NONE;
+	g->known = 0;
+	if (g->kind == FX_NONE) {
+		factor1(m, g);
+		g->known = 1;
+	}
+}
+
 static void load1(const dk_flat_op *op, cpx *m)
 {
 	for (int i = 0; i < 4; i++)
@@ -164,6 +206,7 @@ static void analyse(const dk_flat_op *op, fx_gate *g)
 	g->sup = g->tmask | g->ctl;
 	g->kind = FX_NONE;
 	g->flip = g->unitary = g->is_x = g->gone = 0;
+	g->known = 1;
 	if (op->k > DK_SWEEP_MAX_K)
 		return;
 	if (op->k > 1) {
@@ -178,7 +221,7 @@ static void analyse(const dk_flat_op *op, fx_gate *g)
 	const cpx x = cx(m[0].x * m[1].x + m[0].y * m[1].y + m[2].x * m[3].x + m[2].y * m[3].y,
 			 m[0].x * m[1].y - m[0].y * m[1].x + m[2].x * m[3].y - m[2].y * m[3].x);
 	g->unitary = n0 > 0 && fabsl(n0 - n1) <= 1e-14L * n0 && fabsl(x.x) + fabsl(x.y) <= 1e-14L * n0;
-	factor1(m, g);
+	classify1(m, g);
 	g->is_x = g->kind == FX_PERM && ceq(m[1], c_one) && ceq(m[2], c_one);
 }
 
@@ -1183,8 +1226,9 @@ enum { PUSH_NONE = 0, PUSH_Z, PUSH_X, PUSH_ALL };
 
 /* m as Rx(a) W with W = k [[1, -t], [t, 1]] diag(1, r1), |t| <= 1 (m a
  * multiple of a unitary).  With the first column (A, B): A + B and A - B are
- * multiples of exp(-i a) and exp(i a). */
-static void split_x(const cpx *m, cpx *rx, fx_gate *g)
+ * multiples of exp(-i a) and exp(i a).  0 when t is not real (rx and *g are then
+ * void). */
+static int split_x(const cpx *m, cpx *rx, fx_gate *g)
 {
 	const cpx p = cx(m[0].x + m[2].x, m[0].y + m[2].y), q = cx(m[0].x - m[2].x, m[0].y - m[2].y);
 	cpx z = cx(p.x * q.x + p.y * q.y, p.y * q.x - p.x * q.y), e = c_one; /* exp(-2 i a) */
@@ -1217,16 +1261,24 @@ static void split_x(const cpx *m, cpx *rx, fx_gate *g)
 	g->flip = 0;
 	g->l0 = g->l1 = w[0];
 	g->r1 = r1;
-	g->t = cdiv(w[2], w[0]).x;
-	g->s = -cdiv(w[1], cmul(w[0], r1)).x;
+	const cpx t = cdiv(w[2], w[0]), s = cdiv(w[1], cmul(w[0], r1));
+	g->t = t.x;
+	g->s = -s.x;
+	return fabsl(t.y) <= FX_DROP && fabsl(s.y) <= FX_DROP;
 }
 
 /* A factor on its way from a gate to a later one on the same qubit. */
 typedef struct fx_pending {
 	cpx w[4];
 	int from; /* the gate that gave it, -1: none on its way */
-	fx_gate whole; /* that gate with the factor in it */
+	cpx whole[4]; /* that gate's matrix with the factor in it */
 } fx_pending;
+
+static void set_factors(fx_gate *g, const cpx *m)
+{
+	factor1(m, g);
+	g->known = 1;
+}
 
 /* Moves factors of uncontrolled one-qubit gates to the next such gate on the
  * same qubit, where they join its matrix: the whole gate when nothing on the
@@ -1299,30 +1351,38 @@ static int move_factors(dk_fx_plan *P)
 					t[2 * r + c] = cx(x.x + y.x, x.y + y.y);
 				}
 			fx_gate f = *g;
-			factor1(t, &f);
+			classify1(t, &f);
 			if (f.kind != FX_NONE) {
 				*g = f;
 				memcpy(m, t, sizeof(m));
+				if (!g->known && !push[i])
+					set_factors(g, m);
 			} else {
-				P->g[pd->from] = pd->whole;
+				P->g[pd->from].gone = 0;
+				set_factors(&P->g[pd->from], pd->whole);
 			}
 			pd->from = -1;
 		}
 		if (push[i] == PUSH_NONE)
 			continue;
-		pd->from = i;
-		pd->whole = *g;
+		memcpy(pd->whole, m, sizeof(m));
 		if (push[i] == PUSH_ALL) {
 			memcpy(w, m, sizeof(m));
 			g->gone = 1;
 		} else if (push[i] == PUSH_X) {
-			split_x(m, w, g);
+			if (!split_x(m, w, g)) {
+				set_factors(g, m);
+				continue;
+			}
+			g->known = 1;
 		} else {
+			set_factors(g, m);
 			w[0] = c_one;
 			w[1] = w[2] = cx(0, 0);
 			w[3] = cdiv(g->l1, g->l0);
 			g->l1 = g->l0;
 		}
+		pd->from = i;
 	}
 	free(pend);
 	return DK_OK;
@@ -1373,15 +1433,21 @@ int dk_fx_begin(const dk_flat_op *ops, int nops, unsigned n, int prec,
 	P->nops = 0;
 	for (int i = 0; i < nops; i++) {
 		fx_gate *g = &P->g[i];
+		if (g->gone) {
+			P->ngone++;
+			continue;
+		}
+		if (!g->known) {
+			cpx mt[4];
+			load1(&ops[i], mt);
+			set_factors(g, mt);
+		}
 		g->d0 = cd(g->l0);
 		g->d1 = cd(g->l1);
 		g->dr = cd(g->r1);
 		g->ds = (double)g->s;
 		g->dt = (double)g->t;
-		if (P->g[i].gone)
-			P->ngone++;
-		else
-			P->rem[P->nops++] = i;
+		P->rem[P->nops++] = i;
 	}
 	*out = P;
 	return DK_OK;
