@@ -13,7 +13,9 @@
  * matrices that are not a diagonal times a real rotation) are planned by
  * dk_plan.c.
  *
- * Planning runs while the device works (one step per call), so its cost per
+ * Planning runs while the device works (one step per call): a plan of factored
+ * sweeps only allocates nothing once it has begun, so that it cannot fail between
+ * two sweeps that change a register in place.  For the same reason its cost per
  * gate matters: supports are computed once, a scan ends when every qubit is
  * blocked, and the search for a bank map runs only for sweeps that the fixed
  * residue map leaves with conflicts.
@@ -904,6 +906,12 @@ static void invert4(const uint8_t *rows, uint8_t *cols)
 	}
 }
 
+/* Bytes that a program may have. */
+static size_t program_cap(unsigned n, int m)
+{
+	return n <= (unsigned)m + DK_FX_SMALL_TILES ? DK_FX_BYTES_SMALL : DK_FX_BYTES;
+}
+
 /* Emit the sweep of `cnt` gates (P->take) over Q; gates of passes that no
  * longer fit the program stay in P->take (P->nleft of them). */
 static int emit(dk_fx_plan *P, int cnt, uint64_t Q, int m, dk_step *step,
@@ -1014,7 +1022,7 @@ static int emit(dk_fx_plan *P, int cnt, uint64_t Q, int m, dk_step *step,
 	b->prec = P->prec;
 	b->ncoef = 0;
 	int all_touched = 0, done = 0;
-	const size_t cap = n <= (unsigned)m + DK_FX_SMALL_TILES ? DK_FX_BYTES_SMALL : DK_FX_BYTES;
+	const size_t cap = program_cap(n, m);
 	for (int i = 0; i < npass; i++) {
 		dk_fx_pass *pd = &P->pass[i];
 		const int nop0 = b->nop, nlist0 = b->nlist, ncond0 = b->ncond;
@@ -1390,6 +1398,56 @@ static int move_factors(dk_fx_plan *P)
 
 /* ---- the plan ------------------------------------------------------------- */
 
+/* Most operations and coefficients (doubles) of a gate in a list: a stage emitted
+ * ahead of it (a product or a phase, the rotations along register bits, and one
+ * operation for a rotation of its own), the product behind the stage, its exchange
+ * and two products around its rotation; and of a list's end. */
+#define FX_GATE_OPS 8
+#define FX_GATE_COEFS 200
+#define FX_LIST_OPS 4
+#define FX_LIST_COEFS 90
+
+/* Room for the longest program that the plan can come to: what fits a program, and
+ * the pass that no longer does. */
+static int reserve(dk_fx_plan *P)
+{
+	fx_buf *b = &P->b;
+	const int m = P->lim.tile_bits;
+	const int lists = P->n > (unsigned)m ? 1 << DK_FX_COND : 1; /* of a pass */
+	const size_t cap = program_cap(P->n, m);
+	const size_t gates = (size_t)(P->nops < DK_FX_MAX_GATES ? P->nops : DK_FX_MAX_GATES);
+	const size_t window = gates < FX_WINDOW ? gates : FX_WINDOW;
+	const size_t lops = FX_GATE_OPS * gates + FX_LIST_OPS * gates;
+	const size_t lcoefs = FX_GATE_COEFS * gates + FX_LIST_COEFS * gates;
+	/* a coefficient takes 4 bytes of a program or more */
+	size_t nop = cap / sizeof(dk_fx_op), ncoef = cap / 4, nlist = cap / sizeof(dk_fx_list);
+	if (nop > lops * (size_t)lists)
+		nop = lops * (size_t)lists;
+	if (ncoef > lcoefs * (size_t)lists)
+		ncoef = lcoefs * (size_t)lists;
+	if (nlist > gates * (size_t)lists)
+		nlist = gates * (size_t)lists;
+	size_t bytes = sizeof(dk_sweep_hdr) + sizeof(dk_fx_pass) * gates +
+		       sizeof(dk_fx_list) * nlist + sizeof(dk_fx_op) * nop + 8 * ncoef +
+		       sizeof(b->cond);
+	if (bytes > cap)
+		bytes = cap;
+	nop += (FX_GATE_OPS * window + FX_LIST_OPS) * (size_t)lists;
+	ncoef += (FX_GATE_COEFS * window + FX_LIST_COEFS) * (size_t)lists;
+	nlist += (size_t)lists;
+	b->op = (dk_fx_op *)malloc(sizeof(dk_fx_op) * nop);
+	b->coef = (double *)malloc(sizeof(double) * ncoef);
+	b->list = (dk_fx_list *)malloc(sizeof(dk_fx_list) * nlist);
+	P->prog = (unsigned char *)malloc(bytes);
+	if (!b->op || !b->coef || !b->list || !P->prog)
+		return DK_ERR_ALLOC;
+	b->cop = (int)nop;
+	b->ccoef = ncoef;
+	b->clist = (int)nlist;
+	P->cprog = bytes;
+	return DK_OK;
+}
+
 int dk_fx_begin(const dk_flat_op *ops, int nops, unsigned n, int prec,
 		const dk_plan_limits *lim, dk_fx_plan **out)
 {
@@ -1426,7 +1484,7 @@ int dk_fx_begin(const dk_flat_op *ops, int nops, unsigned n, int prec,
 	}
 	/* gates that dk_plan.c plans from their matrices take no factor */
 	P->all = all;
-	if (all && move_factors(P)) {
+	if (all && (move_factors(P) || reserve(P))) {
 		dk_fx_end(P);
 		return DK_ERR_ALLOC;
 	}

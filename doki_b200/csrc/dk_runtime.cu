@@ -20,6 +20,7 @@
 #include <atomic>
 #include <mutex>
 #include <new>
+#include <utility>
 #include <vector>
 
 #include "dk_internal.h"
@@ -282,38 +283,45 @@ int flush(dk_state *s)
 	}
 }
 
-/* Device copy of `bytes` of host data, valid for work queued on the slot's
- * stream before the slot's next kStagePart bytes.  The host data may be
- * reused when the call returns.  Data larger than a part gets an allocation of
- * its own (*own, freed by the caller after the work that reads it). */
-static int stage_up(const void *src, size_t bytes, const unsigned char **dev, void **own,
-		    size_t *own_bytes)
+/* The staging buffers of the slot, before the first launch of a flush. */
+static int stage_ready()
 {
 	Slot &sl = CUR;
-	*own = nullptr;
+	if (sl.stage_host)
+		return DK_OK;
+	for (int i = 0; i < kStageParts; ++i)
+		if (!sl.copied[i])
+			CK(cudaEventCreateWithFlags(&sl.copied[i], cudaEventDisableTiming));
+	if (!sl.stage_dev)
+		CK(cudaMalloc(&sl.stage_dev, kStagePart * kStageParts));
+	CK(cudaHostAlloc(&sl.stage_host, kStagePart * kStageParts, cudaHostAllocDefault));
+	return DK_OK;
+}
+
+static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
+
+/* Device copy of `bytes` of host data, valid for work queued on the slot's
+ * stream before the slot's next kStagePart bytes.  The host data may be
+ * reused when the call returns.  Data larger than a part goes to the flush's two
+ * places for such data, in turn: when a step is staged, all before the last one
+ * have been launched. */
+struct LargeData {
+	unsigned char *d = nullptr;
+	size_t each = 0; /* bytes of a place */
+	int turn = 0;
+};
+
+static int stage_up(const void *src, size_t bytes, LargeData *large, const unsigned char **dev)
+{
+	Slot &sl = CUR;
 	g.h2d += bytes;
 	if (bytes > kStagePart) {
-		int rc = dev_alloc(own, bytes);
-		if (rc)
-			return rc;
-		*own_bytes = bytes;
-		*dev = (const unsigned char *)*own;
 		/* pageable source: staged before the call returns */
-		cudaError_t e = cudaMemcpyAsync(*own, src, bytes, cudaMemcpyHostToDevice, sl.st);
-		if (e != cudaSuccess) {
-			dev_free(*own, bytes);
-			*own = nullptr;
-			return cuda_fail(e);
-		}
+		unsigned char *const to = large->d + large->each * (size_t)large->turn;
+		CK(cudaMemcpyAsync(to, src, bytes, cudaMemcpyHostToDevice, sl.st));
+		*dev = to;
+		large->turn ^= 1;
 		return DK_OK;
-	}
-	if (!sl.stage_host) {
-		for (int i = 0; i < kStageParts; ++i)
-			if (!sl.copied[i])
-				CK(cudaEventCreateWithFlags(&sl.copied[i], cudaEventDisableTiming));
-		if (!sl.stage_dev)
-			CK(cudaMalloc(&sl.stage_dev, kStagePart * kStageParts));
-		CK(cudaHostAlloc(&sl.stage_host, kStagePart * kStageParts, cudaHostAllocDefault));
 	}
 	size_t at;
 	const int rc = sl.stage.place(
@@ -336,28 +344,59 @@ static int stage_up(const void *src, size_t bytes, const unsigned char **dev, vo
 	return DK_OK;
 }
 
-/* Steps of a flush, from either planner. */
+/* Steps of a flush, from either planner.  A plan of factored sweeps only is made
+ * while the device works: it allocates nothing once it has begun.  Every other
+ * plan is made as a whole before the first launch, so that a host or device
+ * allocation that fails leaves the register as it was. */
 struct StepSource {
-	const std::vector<dk_flat_op> &ops;
 	dk_fx_plan *fx = nullptr;
 	dk_plan plan{};
-	int at = 0;
-	explicit StepSource(const std::vector<dk_flat_op> &o) : ops(o) {}
+	std::vector<dk_step> steps;
+	std::vector<unsigned char> programs;
+	size_t at = 0;
+	bool whole = false;
 	~StepSource()
 	{
 		if (fx)
 			dk_fx_end(fx);
 		dk_plan_free(&plan);
 	}
+	/* Plans everything that cannot wait.  May throw std::bad_alloc. */
+	int prepare()
+	{
+		if (fx && dk_fx_all(fx))
+			return DK_OK;
+		whole = true;
+		if (!fx) {
+			steps.assign(plan.steps, plan.steps + plan.nsteps);
+			return DK_OK;
+		}
+		dk_step step;
+		const unsigned char *prog;
+		int more;
+		while ((more = dk_fx_next(fx, &step, &prog)) > 0) {
+			if (step.kind == 1) {
+				step.prog_off = programs.size();
+				programs.insert(programs.end(), prog,
+						prog + ((const dk_sweep_hdr *)prog)->bytes);
+			}
+			steps.push_back(step);
+		}
+		return -more;
+	}
+	const unsigned char *program(const dk_step &step) const
+	{
+		return step.kind == 1 ? (fx ? programs.data() : plan.blob) + step.prog_off : nullptr;
+	}
 	/* 1: a step, 0: none left, < 0: -status */
 	int next(dk_step *step, const unsigned char **prog)
 	{
-		if (fx)
+		if (!whole)
 			return dk_fx_next(fx, step, prog);
-		if (at >= plan.nsteps)
+		if (at >= steps.size())
 			return 0;
-		*step = plan.steps[at++];
-		*prog = step->kind == 1 ? plan.blob + step->prog_off : nullptr;
+		*step = steps[at++];
+		*prog = program(*step);
 		return 1;
 	}
 };
@@ -370,21 +409,25 @@ struct ReadyStep {
 	dk_sweep_hdr hdr{};
 	unsigned long long entries = 0;
 	const unsigned char *dev = nullptr;
-	void *own = nullptr;
-	size_t own_bytes = 0;
 };
 
+/* The bytes of a step that go to the device. */
+static size_t step_bytes(const std::vector<dk_flat_op> &ops, const dk_step &step,
+			 const unsigned char *prog)
+{
+	if (step.kind == 1)
+		return ((const dk_sweep_hdr *)prog)->bytes;
+	const dk_gate *gt = ops[step.op_index].gate;
+	return 16 * gt->dim * gt->dim;
+}
+
 static int ready_step(const std::vector<dk_flat_op> &ops, unsigned n, const dk_step &step,
-		      const unsigned char *prog, ReadyStep *r)
+		      const unsigned char *prog, LargeData *large, ReadyStep *r)
 {
 	r->step = step;
 	r->entries = 0;
-	const void *src;
-	size_t bytes;
 	if (step.kind == 1) {
 		memcpy(&r->hdr, prog, sizeof(r->hdr));
-		src = prog;
-		bytes = r->hdr.bytes;
 		if (r->hdr.mode == DK_SWEEP_TENSOR) {
 			const dk_pass_desc *pd = (const dk_pass_desc *)(prog + r->hdr.pass_off);
 			for (int p = 0; p < r->hdr.npass; ++p)
@@ -393,12 +436,9 @@ static int ready_step(const std::vector<dk_flat_op> &ops, unsigned n, const dk_s
 			r->entries = (unsigned long long)r->hdr.npass;
 		}
 		r->entries <<= n;
-	} else {
-		const dk_gate *gt = ops[step.op_index].gate;
-		src = gt->m;
-		bytes = 16 * gt->dim * gt->dim;
 	}
-	int rc = stage_up(src, bytes, &r->dev, &r->own, &r->own_bytes);
+	int rc = stage_up(step.kind == 1 ? (const void *)prog : ops[step.op_index].gate->m,
+			  step_bytes(ops, step, prog), large, &r->dev);
 	r->have = rc == DK_OK;
 	return rc;
 }
@@ -437,7 +477,7 @@ static int flush_queued(dk_state *s)
 			(prec == DK_C64 ? g.fx_c64 : g.fx_c128);
 	if (g.low_bits >= 0 && g.low_bits <= lim.tile_bits)
 		lim.low_bits = g.low_bits;
-	StepSource from(ops);
+	StepSource from;
 	int rc = fx ? dk_fx_begin(ops.data(), (int)cnt, n, prec, &lim, &from.fx)
 			 : dk_plan_build(ops.data(), (int)cnt, n, prec, &lim, &from.plan);
 	if (rc)
@@ -455,12 +495,39 @@ static int flush_queued(dk_state *s)
 	if (fx && prec == DK_C64 && n >= 24 && g.low_bits < 0)
 		dk_fx_set_low_bits(from.fx, 4);
 
+	rc = from.prepare();
+	if (rc == DK_OK)
+		rc = stage_ready();
+	if (rc)
+		return rc;
+
+	/* everything that the steps need is allocated before the first of them runs:
+	 * the register's copy where others share the buffer, matrices and programs
+	 * too long for a staging part, the output of generic gates */
 	dk_buf *src = s->buf;
 	dk_buf *dst = src;
-	if (src->refcount > 1) {
+	LargeData large;
+	bool generic = false;
+	for (size_t i = 0; i < from.steps.size(); ++i) {
+		const dk_step &st = from.steps[i];
+		const size_t bytes = step_bytes(ops, st, from.program(st));
+		if (bytes > kStagePart && bytes > large.each)
+			large.each = align256(bytes);
+		/* the first step of a shared register writes the copy */
+		generic |= st.kind == 2 && (i > 0 || src->refcount <= 1);
+	}
+	void *spare = nullptr;
+	if (src->refcount > 1)
 		rc = buf_new(n, prec, &dst);
-		if (rc)
-			return rc;
+	if (rc == DK_OK && large.each)
+		rc = dev_alloc((void **)&large.d, 2 * large.each);
+	if (rc == DK_OK && generic)
+		rc = dev_alloc(&spare, src->bytes);
+	if (rc) {
+		dev_free(large.d, 2 * large.each);
+		if (dst != src)
+			buf_release(dst);
+		return rc;
 	}
 	const void *cur = src->d;
 	const dk_scal *cur_sc = src->sc;
@@ -473,12 +540,12 @@ static int flush_queued(dk_state *s)
 	 * whether a factored sweep must leave its scalars. */
 	int more = from.next(&step, &prog);
 	if (more > 0)
-		rc = ready_step(ops, n, step, prog, &ready);
+		rc = ready_step(ops, n, step, prog, &large, &ready);
 	while (rc == DK_OK && ready.have) {
 		next.have = false;
 		more = from.next(&step, &prog);
 		if (more > 0)
-			rc = ready_step(ops, n, step, prog, &next);
+			rc = ready_step(ops, n, step, prog, &large, &next);
 		else if (more < 0)
 			rc = -more;
 		if (rc)
@@ -503,44 +570,32 @@ static int flush_queued(dk_state *s)
 			g.gates += (unsigned long long)ready.step.ngates;
 		} else {
 			const dk_flat_op &op = ops[ready.step.op_index];
-			void *target = dst->d;
-			void *tmp = nullptr;
-			if (cur == dst->d) {
-				rc = dev_alloc(&tmp, dst->bytes);
-				if (rc)
-					break;
-				target = tmp;
-			}
-			e = dk::launch_generic_gate(prec, cur, target, n, op.k, op.tg,
+			const bool swap = cur == dst->d;
+			e = dk::launch_generic_gate(prec, cur, swap ? spare : dst->d, n, op.k, op.tg,
 						    op.cm, op.am, (const double *)ready.dev,
 						    cur_sc, dst->sc, CUR.scratch, CUR.st);
-			if (tmp) {
-				dev_free(dst->d, dst->bytes);
-				dst->d = tmp;
-			}
+			if (swap)
+				std::swap(dst->d, spare);
 			g.gates++;
 		}
 		if (e != cudaSuccess)
 			rc = cuda_fail(e);
 		cur = dst->d;
 		cur_sc = dst->sc;
-		if (ready.own)
-			dev_free(ready.own, ready.own_bytes);
 		ready = next;
 		next = ReadyStep();
 	}
 	if (rc == DK_OK && more < 0)
 		rc = -more;
-	if (ready.have && ready.own)
-		dev_free(ready.own, ready.own_bytes);
-	if (next.have && next.own)
-		dev_free(next.own, next.own_bytes);
+	dev_free(large.d, 2 * large.each);
+	dev_free(spare, src->bytes);
 	if (rc) {
 		if (dst != src) {
 			buf_release(dst);
 		} else if (launched) {
-			/* some of the gates have already changed the register in
-			 * place: it must not be read, or the rest queued again */
+			/* a CUDA call failed after some of the gates had changed the
+			 * register in place: it must not be read, or the rest queued
+			 * again */
 			op_release(s->pending);
 			s->pending = nullptr;
 			state_drop_caches(s);
