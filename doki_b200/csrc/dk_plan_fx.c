@@ -1484,7 +1484,7 @@ int dk_fx_begin(const dk_flat_op *ops, int nops, unsigned n, int prec,
 	}
 	/* gates that dk_plan.c plans from their matrices take no factor */
 	P->all = all;
-	if (all && (move_factors(P) || reserve(P))) {
+	if ((all && move_factors(P)) || reserve(P)) {
 		dk_fx_end(P);
 		return DK_ERR_ALLOC;
 	}
