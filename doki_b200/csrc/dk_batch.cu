@@ -379,10 +379,10 @@ __global__ void __launch_bounds__(kFxThreads, MINB)
 						return base ^ ((q & 1) ? x & 0xffffu : 0u) ^ ((q & 2) ? x >> 16 : 0u) ^
 						       ((q & 4) ? y & 0xffffu : 0u) ^ ((q & 8) ? y >> 16 : 0u);
 					};
-					const uint32_t gb = sg ^ (l1.x & 0xffffu), sb = sg ^ (l1.x >> 16);
+					const uint32_t sb = sg ^ (l1.x >> 16);
 #pragma unroll
 					for (int q = 0; q < DK_FX_REGS; ++q)
-						a[q] = *reinterpret_cast<const C2 *>(tile + slot(q, gb, l0.x, l0.y));
+						a[q] = *reinterpret_cast<const C2 *>(tile + slot(q, sg, l0.x, l0.y));
 					const uint32_t raw = (ph.x & DK_PASS_CTL)
 								     ? (__ldg(&pd->rlo[lane]) | __ldg(&pd->rhi[warp]))
 								     : 0u;

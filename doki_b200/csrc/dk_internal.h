@@ -250,11 +250,12 @@ typedef struct dk_fx_op {
 
 /* What a pass does where its tile conditions have one combination of values:
  * operations [op0, op1) between a gather and a scatter, whose slots are given
- * by byte offsets for register bit j and for register 0 (relabellings move
- * amplitudes in between, and the gather may choose the labels). */
+ * by byte offsets for register bit j (gt, st) and, for the scatter, for register 0:
+ * relabellings move amplitudes in between, and the gather starts from linear
+ * labels of the planner's choice. */
 typedef struct dk_fx_list {
 	uint16_t gt[DK_FX_BITS], st[DK_FX_BITS];
-	uint16_t gc, sc;
+	uint16_t pad, sc; /* sc: the scatter's offset of register 0; the gather's is 0 */
 	uint16_t op0, op1;
 	/* the scatter as pass indices: L(1 << j) ^ L(0) in nibble j, L(0) in
 	 * nibble 4 (a pass that stores to the register) */

@@ -1117,7 +1117,7 @@ static int emit(dk_fx_plan *P, int cnt, uint64_t Q, int m, dk_step *step,
 					if (cols[j] >> x & 1)
 						gt[j] ^= P->sp[i][x];
 			}
-			li->gc = 0;
+			li->pad = 0;
 			li->op0 = (uint16_t)b->nop;
 			for (int k = 0; k < ng; k++)
 				add_gate(b, &s, &P->ops[gl[k]->id], &P->g[gl[k]->id], gl[k]->treg,

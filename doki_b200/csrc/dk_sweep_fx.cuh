@@ -421,7 +421,7 @@ __device__ __forceinline__ void fx_sweep(const typename CT<R>::T *__restrict__ i
 			if (!l1.w || out_now) {
 				const uint4 l0 = lists[2 * li];
 				const uint32_t sg = pd->slo[lane] ^ pd->shi[warp];
-				read16(sg ^ (l1.x & 0xffffu), l0.x & 0xffffu, l0.x >> 16, l0.y & 0xffffu,
+				read16(sg, l0.x & 0xffffu, l0.x >> 16, l0.y & 0xffffu,
 				       l0.y >> 16);
 				if (out_now) {
 					/* the results of this pass go to the register: once every
