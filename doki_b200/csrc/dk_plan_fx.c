@@ -13,12 +13,12 @@
  * matrices that are not a diagonal times a real rotation) are planned by
  * dk_plan.c.
  *
- * Planning runs while the device works (one step per call): a plan of factored
- * sweeps only allocates nothing once it has begun, so that it cannot fail between
- * two sweeps that change a register in place.  For the same reason its cost per
+ * Planning runs while the device works (one step per call), so its cost per
  * gate matters: supports are computed once, a scan ends when every qubit is
  * blocked, and the search for a bank map runs only for sweeps that the fixed
- * residue map leaves with conflicts.
+ * residue map leaves with conflicts.  Nor may it fail there, between two sweeps
+ * that change a register in place: a plan of factored sweeps only allocates nothing
+ * once dk_fx_reserve has run.
  */
 #include <math.h>
 #include <stdlib.h>
@@ -1217,7 +1217,8 @@ static int emit(dk_fx_plan *P, int cnt, uint64_t Q, int m, dk_step *step,
 	put_coefs(b, P->prec, P->prog + mat_off);
 	memcpy(P->prog + pass_off, P->pass, sizeof(dk_fx_pass) * (size_t)done);
 	memcpy(P->prog + list_off, b->list, sizeof(dk_fx_list) * (size_t)b->nlist);
-	memcpy(P->prog + gate_off, b->op, sizeof(dk_fx_op) * (size_t)b->nop);
+	if (b->nop)
+		memcpy(P->prog + gate_off, b->op, sizeof(dk_fx_op) * (size_t)b->nop);
 	memcpy(P->prog + cond_off, b->cond, sizeof(dk_gate_cond) * (size_t)b->ncond);
 	step->kind = 1;
 	step->prog_off = 0;
@@ -1409,9 +1410,11 @@ static int move_factors(dk_fx_plan *P)
 
 /* Room for the longest program that the plan can come to: what fits a program, and
  * the pass that no longer does. */
-static int reserve(dk_fx_plan *P)
+int dk_fx_reserve(dk_fx_plan *P)
 {
 	fx_buf *b = &P->b;
+	if (b->op || P->prog)
+		return DK_OK; /* reserved before, or steps made without */
 	const int m = P->lim.tile_bits;
 	const int lists = P->n > (unsigned)m ? 1 << DK_FX_COND : 1; /* of a pass */
 	const size_t cap = program_cap(P->n, m);
@@ -1484,7 +1487,7 @@ int dk_fx_begin(const dk_flat_op *ops, int nops, unsigned n, int prec,
 	}
 	/* gates that dk_plan.c plans from their matrices take no factor */
 	P->all = all;
-	if ((all && move_factors(P)) || reserve(P)) {
+	if (all && move_factors(P)) {
 		dk_fx_end(P);
 		return DK_ERR_ALLOC;
 	}

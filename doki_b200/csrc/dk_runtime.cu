@@ -345,7 +345,7 @@ static int stage_up(const void *src, size_t bytes, LargeData *large, const unsig
 }
 
 /* Steps of a flush, from either planner.  A plan of factored sweeps only is made
- * while the device works: it allocates nothing once it has begun.  Every other
+ * while the device works: it has allocated all that it needs by then.  Every other
  * plan is made as a whole before the first launch, so that a host or device
  * allocation that fails leaves the register as it was. */
 struct StepSource {
@@ -365,7 +365,7 @@ struct StepSource {
 	int prepare()
 	{
 		if (fx && dk_fx_all(fx))
-			return DK_OK;
+			return dk_fx_reserve(fx);
 		whole = true;
 		if (!fx) {
 			steps.assign(plan.steps, plan.steps + plan.nsteps);

@@ -113,6 +113,8 @@ int main(int argc, char **argv)
 		for (long k = 0; rc == DK_ERR_ALLOC && k < 100; k++) {
 			left = k;
 			rc = dk_fx_begin(ops, nops, n, prec, &lim, &p);
+			if (rc == 0 && dk_fx_all(p) && (rc = dk_fx_reserve(p)) != 0)
+				dk_fx_end(p);
 			left = -1;
 			begun++;
 		}
