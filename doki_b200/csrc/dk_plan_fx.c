@@ -468,24 +468,34 @@ static void emit_rot(fx_buf *b, const fx_rotn *r, uint32_t lc, uint32_t la)
 		c[i] = !r->plain ? r->co[i] : i >> 1 == __builtin_ctz(r->dir) ? r->co[i & 1] : 0.0;
 }
 
-/* A rotation commutes with a plain one along v: what it adds to a register
- * does not depend on that bit. */
-static int passes_plain(const fx_rotn *r, unsigned v)
+/* What a rotation adds to register p of register p ^ dir. */
+static void rot_coefs(const fx_rotn *r, double *c)
 {
 	const unsigned dir = r->dir, low = dir & (0u - dir);
-	if (r->plain)
-		return 1;
-	double c[DK_FX_REGS];
 	int pr = 0;
 	for (unsigned p = 0; p < DK_FX_REGS; p++) {
 		if (p & low)
 			continue;
-		c[p] = r->co[2 * pr];
-		c[p ^ dir] = r->co[2 * pr + 1];
+		c[p] = r->co[r->plain ? 0 : 2 * pr];
+		c[p ^ dir] = r->co[r->plain ? 1 : 2 * pr + 1];
 		pr++;
 	}
+}
+
+/* Two rotations commute where what each adds to a register is the same along the
+ * other's direction.  (In one order register p gets a[p] b[p ^ dir a] of register
+ * p ^ dir a ^ dir b, in the other b[p] a[p ^ dir b].)  Plain ones along two register
+ * bits do; one along several bits, a CNOT's control and target, say, changes sides
+ * under a plain one along either. */
+static int rots_commute(const fx_rotn *a, const fx_rotn *b)
+{
+	if (a->plain && b->plain && a->dir != b->dir)
+		return 1;
+	double ca[DK_FX_REGS], cb[DK_FX_REGS];
+	rot_coefs(a, ca);
+	rot_coefs(b, cb);
 	for (unsigned p = 0; p < DK_FX_REGS; p++)
-		if (c[p] != c[p ^ v])
+		if (ca[p] != ca[p ^ b->dir] || cb[p] != cb[p ^ a->dir])
 			return 0;
 	return 1;
 }
@@ -502,7 +512,7 @@ static void emit_stage(fx_buf *b, const fx_stage *s)
 		int ahead = s->rot[i].plain && first[j] < 0;
 		for (int k = 0; k < i && ahead; k++)
 			if (rest >> k & 1)
-				ahead = passes_plain(&s->rot[k], s->rot[i].dir);
+				ahead = rots_commute(&s->rot[k], &s->rot[i]);
 		if (ahead) {
 			first[j] = i;
 			mask |= 1u << j;
