@@ -356,6 +356,10 @@ void dk_fx_set_low_bits(dk_fx_plan *p, int low);
  * circuit), so that none of them allocates.  Optional: a plan grows its tables as
  * it needs them otherwise. */
 int dk_fx_reserve(dk_fx_plan *p);
+/* After dk_fx_reserve, and dk_fx_next that failed: the gates (indices of `ops`) that
+ * no step before holds, in an order to apply them in after those steps.  Their number, or -1 for a
+ * plan of factored sweeps only, whose gates have taken factors of others. */
+int dk_fx_left(const dk_fx_plan *p, int *ids);
 /* Every step will be a factored sweep. */
 int dk_fx_all(const dk_fx_plan *p);
 void dk_fx_end(dk_fx_plan *p);

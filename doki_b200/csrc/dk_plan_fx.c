@@ -18,7 +18,8 @@
  * blocked, and the search for a bank map runs only for sweeps that the fixed
  * residue map leaves with conflicts.  Nor may it fail there, between two sweeps
  * that change a register in place: a plan of factored sweeps only allocates nothing
- * once dk_fx_reserve has run.
+ * once dk_fx_reserve has run, and any other plan, whose gates keep the matrices they
+ * were given, can name the gates that it has not come to (dk_fx_left).
  */
 #include <math.h>
 #include <stdlib.h>
@@ -1526,6 +1527,14 @@ int dk_fx_begin(const dk_flat_op *ops, int nops, unsigned n, int prec,
 
 int dk_fx_all(const dk_fx_plan *P) { return P->all; }
 
+int dk_fx_left(const dk_fx_plan *P, int *ids)
+{
+	if (P->all || P->nleft || P->sub_at < P->sub.nsteps)
+		return -1;
+	memcpy(ids, P->rem + P->head, sizeof(int) * (size_t)(P->nops - P->head));
+	return P->nops - P->head;
+}
+
 void dk_fx_set_low_bits(dk_fx_plan *P, int low) { P->low = low; }
 
 void dk_fx_end(dk_fx_plan *P)
@@ -1644,8 +1653,12 @@ int dk_fx_next(dk_fx_plan *P, dk_step *step, const unsigned char **prog)
 			if (P->all)
 				return -DK_ERR_ARG; /* cannot happen: every gate has a factoring */
 			const int rc = sub_plan(P, c.nt);
-			if (rc)
+			if (rc) {
+				/* back in front of what was passed over */
+				P->head -= c.nt;
+				memcpy(P->rem + P->head, P->take, sizeof(int) * (size_t)c.nt);
 				return -rc;
+			}
 			continue;
 		}
 		for (unsigned q = 0; popc(c.Q) < m && q < P->n; q++)

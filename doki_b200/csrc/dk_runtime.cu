@@ -316,6 +316,8 @@ static int stage_up(const void *src, size_t bytes, LargeData *large, const unsig
 	Slot &sl = CUR;
 	g.h2d += bytes;
 	if (bytes > kStagePart) {
+		if (bytes > large->each)
+			return DK_ERR_ALLOC; /* cannot happen: a sweep's program is shorter */
 		/* pageable source: staged before the call returns */
 		unsigned char *const to = large->d + large->each * (size_t)large->turn;
 		CK(cudaMemcpyAsync(to, src, bytes, cudaMemcpyHostToDevice, sl.st));
@@ -344,60 +346,72 @@ static int stage_up(const void *src, size_t bytes, LargeData *large, const unsig
 	return DK_OK;
 }
 
-/* Steps of a flush, from either planner.  A plan of factored sweeps only is made
- * while the device works: it has allocated all that it needs by then.  Every other
- * plan is made as a whole before the first launch, so that a host or device
- * allocation that fails leaves the register as it was. */
+/* Steps of a flush, from either planner. */
 struct StepSource {
 	dk_fx_plan *fx = nullptr;
 	dk_plan plan{};
-	std::vector<dk_step> steps;
-	std::vector<unsigned char> programs;
-	size_t at = 0;
-	bool whole = false;
+	int at = 0;
 	~StepSource()
 	{
 		if (fx)
 			dk_fx_end(fx);
 		dk_plan_free(&plan);
 	}
-	/* Plans everything that cannot wait.  May throw std::bad_alloc. */
-	int prepare()
-	{
-		if (fx && dk_fx_all(fx))
-			return dk_fx_reserve(fx);
-		whole = true;
-		if (!fx) {
-			steps.assign(plan.steps, plan.steps + plan.nsteps);
-			return DK_OK;
-		}
-		dk_step step;
-		const unsigned char *prog;
-		int more;
-		while ((more = dk_fx_next(fx, &step, &prog)) > 0) {
-			if (step.kind == 1) {
-				step.prog_off = programs.size();
-				programs.insert(programs.end(), prog,
-						prog + ((const dk_sweep_hdr *)prog)->bytes);
-			}
-			steps.push_back(step);
-		}
-		return -more;
-	}
-	const unsigned char *program(const dk_step &step) const
-	{
-		return step.kind == 1 ? (fx ? programs.data() : plan.blob) + step.prog_off : nullptr;
-	}
 	/* 1: a step, 0: none left, < 0: -status */
 	int next(dk_step *step, const unsigned char **prog)
 	{
-		if (!whole)
+		if (fx)
 			return dk_fx_next(fx, step, prog);
-		if (at >= steps.size())
+		if (at >= plan.nsteps)
 			return 0;
-		*step = steps[at++];
-		*prog = program(*step);
+		*step = plan.steps[at++];
+		*prog = step->kind == 1 ? plan.blob + step->prog_off : nullptr;
 		return 1;
+	}
+};
+
+/* Nodes for the gates that a flush may have to queue again, one per gate. */
+struct SpareOps {
+	std::vector<dk_op *> node;
+	std::vector<int> ids;
+	~SpareOps()
+	{
+		for (dk_op *o : node)
+			free(o);
+	}
+	/* May throw std::bad_alloc. */
+	int make(size_t count)
+	{
+		ids.resize(count);
+		node.reserve(count);
+		for (size_t i = 0; i < count; ++i) {
+			dk_op *o = (dk_op *)calloc(1, sizeof(dk_op));
+			if (!o)
+				return DK_ERR_ALLOC;
+			node.push_back(o);
+		}
+		return DK_OK;
+	}
+	/* The gates ids[0 .. count) as a chain, which takes their nodes. */
+	dk_op *chain(const std::vector<dk_flat_op> &ops, int count)
+	{
+		dk_op *last = nullptr;
+		for (int i = 0; i < count; ++i) {
+			const dk_flat_op &f = ops[ids[i]];
+			dk_op *o = node[i];
+			node[i] = nullptr;
+			o->refcount = 1;
+			o->prev = last;
+			o->gate = const_cast<dk_gate *>(f.gate);
+			gate_retain(o->gate);
+			o->k = f.k;
+			memcpy(o->tg, f.tg, sizeof(o->tg));
+			o->cm = f.cm;
+			o->am = f.am;
+			o->depth = (uint32_t)i + 1;
+			last = o;
+		}
+		return last;
 	}
 };
 
@@ -495,26 +509,35 @@ static int flush_queued(dk_state *s)
 	if (fx && prec == DK_C64 && n >= 24 && g.low_bits < 0)
 		dk_fx_set_low_bits(from.fx, 4);
 
-	rc = from.prepare();
+	/* Sweeps change the register in place while later ones are planned, and a
+	 * failed allocation must leave it as it was.  A plan of factored sweeps only
+	 * has all that it needs from here on.  Another plan may fail on the way; the
+	 * gates that it has not come to are then queued again. */
+	SpareOps again;
+	if (fx)
+		rc = dk_fx_reserve(from.fx);
+	if (rc == DK_OK && fx && !dk_fx_all(from.fx))
+		rc = again.make(cnt);
 	if (rc == DK_OK)
 		rc = stage_ready();
 	if (rc)
 		return rc;
 
-	/* everything that the steps need is allocated before the first of them runs:
-	 * the register's copy where others share the buffer, matrices and programs
-	 * too long for a staging part, the output of generic gates */
+	/* the device memory of all steps: the register's copy where others share the
+	 * buffer, and for gates that no sweep runs their output and the matrices too
+	 * long for a staging part */
 	dk_buf *src = s->buf;
 	dk_buf *dst = src;
 	LargeData large;
 	bool generic = false;
-	for (size_t i = 0; i < from.steps.size(); ++i) {
-		const dk_step &st = from.steps[i];
-		const size_t bytes = step_bytes(ops, st, from.program(st));
+	for (uint32_t i = 0; i < cnt; ++i) {
+		if (ops[i].k <= DK_SWEEP_MAX_K && lim.tile_bits >= DK_PASS_BITS)
+			continue;
+		const size_t bytes = 16 * ops[i].gate->dim * ops[i].gate->dim;
 		if (bytes > kStagePart && bytes > large.each)
 			large.each = align256(bytes);
-		/* the first step of a shared register writes the copy */
-		generic |= st.kind == 2 && (i > 0 || src->refcount <= 1);
+		/* as the first step it writes the copy of a shared register */
+		generic |= i > 0 || src->refcount <= 1;
 	}
 	void *spare = nullptr;
 	if (src->refcount > 1)
@@ -546,9 +569,9 @@ static int flush_queued(dk_state *s)
 		more = from.next(&step, &prog);
 		if (more > 0)
 			rc = ready_step(ops, n, step, prog, &large, &next);
-		else if (more < 0)
-			rc = -more;
-		if (rc)
+		/* a plan that has failed: what it has made still runs if the register
+		 * has begun to change */
+		if (rc || (more < 0 && !launched))
 			break;
 		cudaError_t e;
 		launched = true;
@@ -585,7 +608,8 @@ static int flush_queued(dk_state *s)
 		ready = next;
 		next = ReadyStep();
 	}
-	if (rc == DK_OK && more < 0)
+	const bool planned = rc == DK_OK && more < 0; /* all that was planned has run */
+	if (planned)
 		rc = -more;
 	dev_free(large.d, 2 * large.each);
 	dev_free(spare, src->bytes);
@@ -593,13 +617,15 @@ static int flush_queued(dk_state *s)
 		if (dst != src) {
 			buf_release(dst);
 		} else if (launched) {
-			/* a CUDA call failed after some of the gates had changed the
-			 * register in place: it must not be read, or the rest queued
-			 * again */
+			/* the gates that have run are done with; the others are queued
+			 * again, unless a CUDA call failed and no one knows which those
+			 * are: then the register must not be read any more */
+			const int left = planned && fx ? dk_fx_left(from.fx, again.ids.data()) : -1;
+			dk_op *const rest = left > 0 ? again.chain(ops, left) : nullptr;
 			op_release(s->pending);
-			s->pending = nullptr;
+			s->pending = rest;
 			state_drop_caches(s);
-			s->released = 1;
+			s->released = left < 0;
 		}
 		return rc;
 	}

@@ -1,6 +1,7 @@
 """Many large gate matrices in one flush: they pass through a ring of two 1 MiB
 parts on their way to the device while the gates before them run.  8-qubit matrices
-fill a part exactly, 7- and 4-qubit ones after 4 and 256.  Compared with the same
+fill a part exactly, 7- and 4-qubit ones after 4 and 256, 9-qubit ones are longer
+than a part.  Compared with the same
 gates flushed one at a time (the same kernels on the same data: equal to the last
 bit)."""
 from __future__ import annotations
@@ -14,7 +15,7 @@ from tests.golden.gen_golden import random_unitary
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("n,k,count", [(24, 8, 7), (22, 7, 20), (20, 4, 600)])
+@pytest.mark.parametrize("n,k,count", [(24, 8, 7), (22, 7, 20), (20, 4, 600), (20, 9, 6)])
 def test_matrices_in_one_flush(dk_gpu, n, k, count):
     d = dk_gpu
     rng = W.rng_for(60 + k)

@@ -1,8 +1,8 @@
 """Host allocation failures in the factored-sweep planner (doki_b200/csrc/dk_plan_fx.c),
 on CPU: a C driver in which allocations fail on demand.  Sweeps change a register in
 place while the next ones are planned, so a plan of factored sweeps may fail when it
-begins and not later; a plan with other sweeps in it fails with a status at any
-step.  Under AddressSanitizer: nothing is lost or used again on the way."""
+begins and not later; a plan with other sweeps in it may fail at any step and then
+names the gates that are left.  Under AddressSanitizer: nothing is lost or used again on the way."""
 from __future__ import annotations
 
 import os
@@ -64,6 +64,14 @@ static struct dk_gate *make(unsigned k, int kind)
 			m[e] = cos(angle());
 	}
 	return g;
+}
+
+static uint64_t support(const dk_flat_op *op)
+{
+	uint64_t s = op->cm | op->am;
+	for (unsigned j = 0; j < op->k; j++)
+		s |= 1ull << op->tg[j];
+	return s;
 }
 
 int main(int argc, char **argv)
@@ -138,6 +146,9 @@ int main(int argc, char **argv)
 				return 4;
 			}
 		} else {
+			const int reserved = below(4) != 0;
+			if (reserved && dk_fx_reserve(p))
+				return 12;
 			left = (long)below(60);
 			while ((rc = dk_fx_next(p, &step, &prog)) > 0)
 				gates_done += step.kind == 1 ? step.ngates : 1;
@@ -145,6 +156,27 @@ int main(int argc, char **argv)
 			if (rc != 0 && rc != -DK_ERR_ALLOC)
 				return 5;
 			refused += rc != 0;
+			/* what is left after a failure: every gate that no step holds, after
+			 * all gates before it that it depends on */
+			int *ids = __real_calloc((size_t)nops, sizeof(int));
+			char *in = __real_calloc((size_t)nops, 1);
+			const int rest = rc && reserved ? dk_fx_left(p, ids) : 0;
+			if (rest < 0 || ((!rc || reserved) && gates_done + rest != nops))
+				return 6;
+			for (int i = 0; i < rest; i++) {
+				if (ids[i] < 0 || ids[i] >= nops || in[ids[i]]++)
+					return 7;
+				const uint64_t si = support(&ops[ids[i]]);
+				for (int j = 0; j < i; j++)
+					if (ids[j] > ids[i] && support(&ops[ids[j]]) & si)
+						return 8;
+			}
+			for (int i = 0; i < rest; i++)
+				for (int j = ids[i] + 1; j < nops; j++)
+					if (rest && !in[j] && support(&ops[j]) & support(&ops[ids[i]]))
+						return 9; /* j ran before a gate that it comes after */
+			free(ids);
+			free(in);
 		}
 		dk_fx_end(p);
 		for (int i = 0; i < nops; i++) {
