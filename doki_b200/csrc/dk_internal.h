@@ -349,9 +349,6 @@ typedef struct dk_fx_plan dk_fx_plan;
 int dk_fx_begin(const dk_flat_op *ops, int nops, unsigned n, int prec,
 		const dk_plan_limits *lim, dk_fx_plan **out);
 int dk_fx_next(dk_fx_plan *p, dk_step *step, const unsigned char **prog);
-/* Qubits that are always in a factored sweep's tile, instead of the limits'
- * low_bits, which the other sweeps keep.  Before the first step. */
-void dk_fx_set_low_bits(dk_fx_plan *p, int low);
 /* Allocates the most that the factored steps can need (about 1 MiB for a long
  * circuit), so that none of them allocates.  Optional: a plan grows its tables as
  * it needs them otherwise. */

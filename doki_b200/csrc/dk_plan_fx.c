@@ -253,7 +253,6 @@ struct dk_fx_plan {
 	int ngone; /* gates absorbed by others, not yet counted in a step */
 	int all; /* every gate has a factoring */
 	dk_plan_limits lim;
-	int low; /* qubits always in the tile of a factored sweep */
 	int *rem, head; /* gates left: rem[head .. nops) */
 	int *take, *order, *win; /* a sweep's gates; in pass order; a pass's leftovers */
 	dk_fx_pass *pass;
@@ -1473,7 +1472,6 @@ int dk_fx_begin(const dk_flat_op *ops, int nops, unsigned n, int prec,
 	P->n = n;
 	P->prec = prec;
 	P->lim = *lim;
-	P->low = lim->low_bits;
 	P->cpass = DK_MAX_FX_PASSES;
 	const size_t cnt = (size_t)(nops > 0 ? nops : 1);
 	P->g = (fx_gate *)calloc(cnt, sizeof(fx_gate));
@@ -1535,8 +1533,6 @@ int dk_fx_left(const dk_fx_plan *P, int *ids)
 	return P->nops - P->head;
 }
 
-void dk_fx_set_low_bits(dk_fx_plan *P, int low) { P->low = low; }
-
 void dk_fx_end(dk_fx_plan *P)
 {
 	if (!P)
@@ -1585,9 +1581,10 @@ typedef struct fx_choice {
 	int factored;
 } fx_choice;
 
-static fx_choice choose(dk_fx_plan *P, int low)
+static fx_choice choose(dk_fx_plan *P)
 {
 	const int m = P->lim.tile_bits;
+	int low = P->lim.low_bits;
 	if (low > m - DK_SWEEP_MAX_K)
 		low = m - DK_SWEEP_MAX_K;
 	uint64_t Q = (UINT64_C(1) << (low > 0 ? low : 0)) - 1u, blocked = 0;
@@ -1640,10 +1637,7 @@ int dk_fx_next(dk_fx_plan *P, dk_step *step, const unsigned char **prog)
 		}
 		if (P->head >= P->nops)
 			return 0;
-		fx_choice c = choose(P, P->low);
-		/* the pinned low qubits are those of the sweep that will run */
-		if (!c.factored && P->low != P->lim.low_bits)
-			c = choose(P, P->lim.low_bits);
+		fx_choice c = choose(P);
 		/* what was passed over comes right before what was not looked at */
 		P->head = c.end - c.nd;
 		memcpy(P->rem + P->head, P->order, sizeof(int) * (size_t)c.nd);

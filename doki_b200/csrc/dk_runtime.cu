@@ -489,6 +489,18 @@ static int flush_queued(dk_state *s)
 	lim.bank_mode = (prec == DK_C64 && dk::g_c64_tmem) ? 1 : 0;
 	const bool fx = lim.tensor > 0 && g.fuse && lim.tile_bits >= DK_FX_MIN_TILE &&
 			(prec == DK_C64 ? g.fx_c64 : g.fx_c128);
+	/* Factored complex64 sweeps pin 4 low qubits (128-byte runs, as complex128
+	 * sweeps pin 2 for 64-byte ones): at 28 qubits, depth 20, 36 and 34 sweeps
+	 * (brickwork, random pairs) in 59.5 and 56.7 ms against 30 and 29 sweeps in
+	 * 60.4 and 61.3 ms with 2 pinned.  complex128: 97.2 and 97.5 ms with 2,
+	 * 101.3 and 96.9 with 3, 101.2 and 97.5 with 4.  A register that stays in the
+	 * L2 cache (below 24 qubits) gains nothing from longer runs.
+	 * The tensor sweeps of dense gates take the same runs: more sweeps (brickwork,
+	 * depth 20: 28 for 21 at 24 qubits, 31 for 25 at 28) that stream faster.  Time
+	 * with 4 against 2 pinned: 24 qubits 1.02 to 1.12, 25 0.95 to 1.05, 26 to 28
+	 * 0.90 to 1.00, 29 0.94 to 1.07; among factored sweeps 0.92 (24) and 0.97 (28). */
+	if (fx && prec == DK_C64 && n >= 24)
+		lim.low_bits = 4;
 	if (g.low_bits >= 0 && g.low_bits <= lim.tile_bits)
 		lim.low_bits = g.low_bits;
 	StepSource from;
@@ -496,19 +508,6 @@ static int flush_queued(dk_state *s)
 			 : dk_plan_build(ops.data(), (int)cnt, n, prec, &lim, &from.plan);
 	if (rc)
 		return rc;
-	/* Factored complex64 sweeps pin 4 low qubits (128-byte runs, as complex128
-	 * sweeps pin 2 for 64-byte ones): at 28 qubits, depth 20, 36 and 34 sweeps
-	 * (brickwork, random pairs) in 59.5 and 56.7 ms against 30 and 29 sweeps in
-	 * 60.4 and 61.3 ms with 2 pinned.  complex128: 97.2 and 97.5 ms with 2,
-	 * 101.3 and 96.9 with 3, 101.2 and 97.5 with 4.  A register that stays in the
-	 * L2 cache (below 24 qubits) gains nothing from longer runs.  The tensor
-	 * sweeps of dense gates keep 2: 4 give them more sweeps (brickwork, depth 20,
-	 * 28 for 21 at 24 qubits, 31 for 25 at 28) and no gain over all sizes, times
-	 * with 4 against 2: 24 qubits 2 to 11 % longer, 28 2 to 10 % shorter, 29 from
-	 * 6 % longer to 6 % shorter. */
-	if (fx && prec == DK_C64 && n >= 24 && g.low_bits < 0)
-		dk_fx_set_low_bits(from.fx, 4);
-
 	/* Sweeps change the register in place while later ones are planned, and a
 	 * failed allocation must leave it as it was.  A plan of factored sweeps only
 	 * has all that it needs from here on.  Another plan may fail on the way; the

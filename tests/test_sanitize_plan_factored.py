@@ -97,8 +97,6 @@ STEPS = """		if (t & 1)
 					unitary(gates[i]);
 		dk_fx_plan *plan = NULL;
 		int rc = dk_fx_begin(ops, nops, n, prec, &lim, &plan);
-		if (rc == 0 && below(2))
-			dk_fx_set_low_bits(plan, (int)below((unsigned)lim.tile_bits + 1));
 		long done = 0;
 		dk_step step;
 		const unsigned char *prog = NULL;
